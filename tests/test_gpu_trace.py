@@ -248,3 +248,52 @@ def test_degenerate_and_coincident_triangles(wr_lib, oracle_lib, tmp_path):
     assert np.isfinite(img).all() and img.mean() > 0
     lo, hi = osc.trace_occluded_bracket(rays)
     assert_within_bracket(occ, lo, hi)
+
+
+def _nested_quads(n, ratio):
+    """A tree that is as deep as it is long: quads across the x axis at ratio^i, half as wide as far
+    from the origin, and a light above the first."""
+    from wurstrenderer_b200 import scenes
+    spec = scenes.SceneSpec()
+    grey = scenes.Material("m_grey", kd=(0.5, 0.5, 0.5))
+    for i in range(n):
+        x = ratio ** i
+        p, t = scenes.quad((x, -x / 2, -x / 2), (x * 1.01, x / 2, -x / 2), (x * 1.01, x / 2, x / 2), (x, -x / 2, x / 2))
+        spec.add("q%03d" % i, grey, p, t)
+    p, t = scenes.quad((1.2, 2.0, -0.2), (1.6, 2.0, -0.2), (1.6, 2.0, 0.2), (1.2, 2.0, 0.2))
+    spec.add("light", scenes.Material("m_light", ke=(5.0, 5.0, 5.0)), p, t)
+    return spec
+
+
+@pytest.mark.parametrize("builder", [0, 1])
+@pytest.mark.parametrize("n,ratio", [(1, 0.5), (2, 0.5), (40, 0.6), (60, 0.5)])
+def test_deep_trees_and_the_stack(wr_lib, tmp_path, n, ratio, builder):
+    """Shallow and very deep trees: a ray's answer does not depend on the rays beside it (each
+    thread's stack is its own), and every block size of the traversal renders the same image."""
+    from wurstrenderer_b200 import scenes
+    cam = {"pos": [2.5, 0.6, 0.7], "lookat": [0.0, 0.0, 0.0], "up": [0.0, 1.0, 0.0], "fovy": 50.0}
+    path = scenes.write_spec(str(tmp_path), "nested", _nested_quads(n, ratio), cam, [40, 30], 4, 6)
+    rng = np.random.default_rng(n)
+    m = 4001
+    rays = np.zeros((m, 8), np.float32)
+    rays[:, 0:3] = rng.uniform(-1.0, 2.0, (m, 3))
+    rays[::3, 0] = 2.0      # down the chain, near its axis
+    rays[::3, 1:3] *= 0.05
+    tgt = np.zeros((m, 3))
+    tgt[:, 0] = ratio ** rng.uniform(0, n, m)
+    d = tgt - rays[:, 0:3] + 0.2 * tgt[:, :1] * rng.uniform(-1, 1, (m, 3))
+    rays[:, 4:7] = d / np.linalg.norm(d, axis=1, keepdims=True)
+    rays[:, 3], rays[:, 7] = 1e-4, np.inf
+    order = rng.permutation(m)
+    with wr_lib.Scene.from_file(path, bvh_builder=builder) as sc:
+        assert sc.info["bvh_depth"] > (20 if n == 60 and builder == 0 else 0)
+        hits, other = sc.trace_closest(rays), sc.trace_closest(rays[order])
+        occ, occ_other = sc.trace_occluded(rays), sc.trace_occluded(rays[order])
+        images = [sc.render(spp=4, seed=3, trace_block=b) for b in (64, 128, 256)]
+        images.append(sc.render(spp=4, seed=3, use_graph=False, profile=2))
+    for a, b in zip(hits, other):
+        assert np.array_equal(a[order], b)
+    assert np.array_equal(occ[order], occ_other)
+    assert np.array_equal(occ != 0, hits[0] >= 0)
+    for im in images[1:]:
+        assert np.allclose(im, images[0], rtol=1e-9, atol=1e-12)

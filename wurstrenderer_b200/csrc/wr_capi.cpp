@@ -389,6 +389,8 @@ void build_device_scene(wr_scene &s) {
     wrd::DevScene &d = s.dev;
     d.nodes = wide ? nullptr : s.nodes.as<float4>();
     d.wnodes = wide ? s.wnodes.as<uint4>() : nullptr;
+    // a ray pushes at most one entry per level of the tree; one more for the sentinel
+    d.stack_words = bvh.depth + 2;
     d.tris = s.tris.as<float4>();
     d.patches = npatch ? s.patches.as<double>() : nullptr;
     d.tri_mat = s.tri_mat.as<uint32_t>();
@@ -628,8 +630,8 @@ void render_jobs(wr_scene &s, const std::vector<HostJob> &jobs, const wr_render_
     if (desc.max_iterations < 0) throw Error(WR_ERR_INVALID_ARGUMENT, "max_iterations must be >= 0");
     if (desc.max_iterations > 0) r.iter_limit = std::min(r.iter_limit, uint32_t(desc.max_iterations));
     r.trace_block = (desc.trace_block == 64 || desc.trace_block == 256) ? desc.trace_block : 128;
-    r.grid_trace = desc.grid_trace > 0 ? desc.grid_trace : sms * std::max(1, wrk::occupancy_blocks(0, r.trace_block, s.dev.patches != nullptr, s.dev.wnodes != nullptr));
-    r.grid_shade = desc.grid_shade > 0 ? desc.grid_shade : sms * std::max(1, wrk::occupancy_blocks(1));
+    r.grid_trace = desc.grid_trace > 0 ? desc.grid_trace : sms * std::max(1, wrk::trace_occupancy(s.dev, r.trace_block));
+    r.grid_shade = desc.grid_shade > 0 ? desc.grid_shade : sms * std::max(1, wrk::shade_occupancy());
 
     const int profile = desc.profile;
     s.w_prof.alloc(16 * 8);
@@ -1388,8 +1390,8 @@ wr_render_desc tune_knobs(wr_scene &s, wr_render_desc cur, Probe probe, double *
     }
     // 3) persistent-CTA count of the traversal and shading kernels
     const int blk = (cur.trace_block == 64 || cur.trace_block == 256) ? cur.trace_block : 128;
-    const int occ_t = sms * std::max(1, wrk::occupancy_blocks(0, blk, s.dev.patches != nullptr, s.dev.wnodes != nullptr));
-    const int occ_s = sms * std::max(1, wrk::occupancy_blocks(1));
+    const int occ_t = sms * std::max(1, wrk::trace_occupancy(s.dev, blk));
+    const int occ_s = sms * std::max(1, wrk::shade_occupancy());
     for (double f : {0.5, 1.0}) {
         wr_render_desc d = cur;
         d.grid_trace = std::max(sms, int(occ_t * f));

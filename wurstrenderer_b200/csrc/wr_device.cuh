@@ -30,8 +30,7 @@ constexpr float kRayEps = 1e-4f;              // Ray<Vec>::Epsilon (src/common/m
 
 constexpr int kTraceBlock = 128;   // threads per block of the traversal kernels
 constexpr int kShadeBlock = 256;   // threads per block of shade / raygen
-constexpr int kSmemStack = 8;      // traversal stack entries kept in shared memory per ray (the rest in local memory)
-constexpr int kMaxStack = 64;      // total traversal stack entries (the BVH builder stays below)
+constexpr int kMaxStack = 64;      // deepest tree that the traversal stack takes (the BVH builders stay below)
 
 // device counters of the wavefront loop (uint32 each)
 enum Counter {
@@ -98,6 +97,7 @@ struct DevScene {
     const float4 *tris;             // leaf order: p0, p1, p2 (.w: index | patch flag, mesh, primitive)
     const double *patches;          // Phong tessellation patches (wrp::kPatchDoubles per leaf primitive),
                                     // nullptr when the scene has none
+    int stack_words;                // traversal stack entries per thread (the tree's depth and the sentinel)
     const uint32_t *tri_mat;
     const DevMaterial *materials;
     const DevLight *lights;

@@ -383,14 +383,13 @@ __device__ __forceinline__ void film_add(const WaveArgs &w, uint32_t slot, f3 c)
 //   count_ctr: the counter holding the queue length (CTR_ACTIVE; CTR_SHADOW, or
 //              CTR_SHADOW_PENDING for the previous iteration's queue)
 
-template <int BLOCK, bool SHADOW, bool PHONG, bool WIDE>
+//   COUNT: node visits and triangle tests are counted into w.prof (profiled renders)
+template <int BLOCK, bool SHADOW, bool PHONG, bool WIDE, bool COUNT>
 __device__ __forceinline__ void trace_queue(const DevScene &s, const WaveArgs &w, uint32_t *stack, int count_ctr) {
     const uint32_t n = SHADOW ? min(w.ctr[count_ctr], w.shadow_capacity) : w.ctr[count_ctr];
     uint32_t *fetch = w.ctr + (SHADOW ? CTR_SHADOW_FETCH : CTR_EXTEND_FETCH);
     TraceStack st;
-    st.smem = stack + threadIdx.x;
-    st.stride = BLOCK;
-    st.sp = 0;
+    st.init(stack + threadIdx.x, BLOCK);
     RayPre r{};
     PatchRay pr{};   // read only by the PHONG instantiation
     float t = 0.f, bu = 0.f, bv = 0.f;
@@ -421,7 +420,7 @@ __device__ __forceinline__ void trace_queue(const DevScene &s, const WaveArgs &w
                         oct = ray_octant(xyz(d));
                     }
                     t = tmax; tri = MISS; bu = 0.f; bv = 0.f;
-                    node = 0; leaf = 0; st.sp = 0;
+                    node = 0; leaf = 0; st.clear();
                     busy = true;
                 } else {
                     exhausted = true;   // the queue counter only grows: no lane gets another ray
@@ -433,11 +432,11 @@ __device__ __forceinline__ void trace_queue(const DevScene &s, const WaveArgs &w
         bool finished = false;
         if (busy) {
             if (WIDE)
-                finished = traverse_steps_w8<SHADOW, PHONG>(s.wnodes, s.tris, r, oct, kRayEps, t, tri, bu, bv, ws, st,
+                finished = traverse_steps_w8<SHADOW, PHONG, false, COUNT>(s.wnodes, s.tris, r, oct, kRayEps, t, tri, bu, bv, ws, st,
                                                              nv, nt, min_active, s.patches, pr);
             else
-                finished = traverse_steps<SHADOW, PHONG>(s.nodes, s.tris, r, kRayEps, t, tri, bu, bv, node, leaf, st,
-                                                          nv, nt, min_active, s.patches, pr);
+                finished = traverse_steps<SHADOW, PHONG, false, COUNT>(s.nodes, s.tris, r, kRayEps, t, tri, bu, bv, node, leaf,
+                                                                       st, nv, nt, min_active, s.patches, pr);
         }
         if (finished) {
             busy = false;
@@ -452,7 +451,7 @@ __device__ __forceinline__ void trace_queue(const DevScene &s, const WaveArgs &w
             }
         }
     }
-    if (w.prof) {   // the whole warp leaves the loop together: one atomic per warp and counter
+    if (COUNT) {   // the whole warp leaves the loop together: one atomic per warp and counter
         const uint32_t wnv = __reduce_add_sync(0xffffffffu, nv), wnt = __reduce_add_sync(0xffffffffu, nt);
         if (lane == 0) {
             atomicAdd(w.prof + (SHADOW ? 8 : 6), (unsigned long long)wnv);
@@ -462,10 +461,11 @@ __device__ __forceinline__ void trace_queue(const DevScene &s, const WaveArgs &w
     }
 }
 
-template <int BLOCK, bool PHONG, bool WIDE>
+// dynamic shared memory of the traversal kernels: DevScene::stack_words x BLOCK words
+template <int BLOCK, bool PHONG, bool WIDE, bool COUNT>
 __global__ void __launch_bounds__(BLOCK) k_extend(DevScene s, WaveArgs w) {
-    __shared__ uint32_t stack[kSmemStack * BLOCK];
-    trace_queue<BLOCK, false, PHONG, WIDE>(s, w, stack, CTR_ACTIVE);
+    extern __shared__ uint32_t stack[];
+    trace_queue<BLOCK, false, PHONG, WIDE, COUNT>(s, w, stack, CTR_ACTIVE);
 }
 
 // lens point of a sample's camera vertex (ThinlensCamera::sampleWe0ByPdf, thinlens.h:121-136; the
@@ -939,10 +939,10 @@ __global__ void __launch_bounds__(kShadeBlock) k_raygen(DevScene s, WaveArgs w) 
     }
 }
 
-template <int BLOCK, bool PHONG, bool WIDE>
+template <int BLOCK, bool PHONG, bool WIDE, bool COUNT>
 __global__ void __launch_bounds__(BLOCK) k_shadow(DevScene s, WaveArgs w, int count_ctr) {
-    __shared__ uint32_t stack[kSmemStack * BLOCK];
-    trace_queue<BLOCK, true, PHONG, WIDE>(s, w, stack, count_ctr);
+    extern __shared__ uint32_t stack[];
+    trace_queue<BLOCK, true, PHONG, WIDE, COUNT>(s, w, stack, count_ctr);
 }
 
 // Extend of this iteration and the shadow rays of the previous one in one persistent launch:
@@ -951,23 +951,23 @@ __global__ void __launch_bounds__(BLOCK) k_shadow(DevScene s, WaveArgs w, int co
 // queues are independent: extend reads this wavefront's rays and writes hit records; the
 // shadow rays were queued by the previous shade / raygen and only add to the film (the next
 // shade appends to the shadow queue only after this launch).
-template <int BLOCK, bool PHONG, bool WIDE>
+template <int BLOCK, bool PHONG, bool WIDE, bool COUNT>
 __device__ __forceinline__ void trace_pair(const DevScene &s, const WaveArgs &w) {
-    __shared__ uint32_t stack[kSmemStack * BLOCK];
-    trace_queue<BLOCK, false, PHONG, WIDE>(s, w, stack, CTR_ACTIVE);
-    trace_queue<BLOCK, true, PHONG, WIDE>(s, w, stack, CTR_SHADOW_PENDING);
+    extern __shared__ uint32_t stack[];
+    trace_queue<BLOCK, false, PHONG, WIDE, COUNT>(s, w, stack, CTR_ACTIVE);
+    trace_queue<BLOCK, true, PHONG, WIDE, COUNT>(s, w, stack, CTR_SHADOW_PENDING);
 }
 
-template <int BLOCK, bool WIDE>
+template <int BLOCK, bool WIDE, bool COUNT>
 __global__ void __launch_bounds__(BLOCK) k_trace_pair(DevScene s, WaveArgs w) {
-    trace_pair<BLOCK, false, WIDE>(s, w);
+    trace_pair<BLOCK, false, WIDE, COUNT>(s, w);
 }
 
 // With Phong patches both FP64 patch tests in one kernel would take 190 registers (2 blocks of
 // 128 per SM); the bound keeps the 384 resident threads per SM of the separate kernels.
-template <int BLOCK, bool WIDE>
+template <int BLOCK, bool WIDE, bool COUNT>
 __global__ void __launch_bounds__(BLOCK, (384 / BLOCK > 0 ? 384 / BLOCK : 1)) k_trace_pair_phong(DevScene s, WaveArgs w) {
-    trace_pair<BLOCK, true, WIDE>(s, w);
+    trace_pair<BLOCK, true, WIDE, COUNT>(s, w);
 }
 
 // queue bookkeeping between iterations (one thread); also drives the graph's while loop
@@ -1019,7 +1019,9 @@ __global__ void k_resolve(const double *film, double *out, uint32_t total_pix, c
 template <bool PHONG, bool WIDE>
 __global__ void __launch_bounds__(kTraceBlock) k_trace_batch(DevScene s, const float4 *rays, uint32_t n, int any_hit,
                                                            float4 *out, uint32_t *visits) {
-    __shared__ uint32_t stack[kSmemStack * kTraceBlock];
+    extern __shared__ uint32_t stack[];
+    TraceStack st;
+    st.init(stack + threadIdx.x, kTraceBlock);
     uint32_t nv = 0, nt = 0;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const float4 a = rays[2 * i], b = rays[2 * i + 1];
@@ -1027,16 +1029,16 @@ __global__ void __launch_bounds__(kTraceBlock) k_trace_batch(DevScene s, const f
         uint32_t tri;
         bool hit;
         if (WIDE && any_hit)
-            hit = traverse_w8<true, PHONG>(s.wnodes, s.tris, xyz(a), xyz(b), a.w, b.w, stack, t, tri, bu, bv, &nv,
-                                           &nt, s.patches);
+            hit = traverse_w8<true, PHONG>(s.wnodes, s.tris, xyz(a), xyz(b), a.w, b.w, st, t, tri, bu, bv, nv, nt,
+                                           s.patches);
         else if (WIDE)
-            hit = traverse_w8<false, PHONG>(s.wnodes, s.tris, xyz(a), xyz(b), a.w, b.w, stack, t, tri, bu, bv, &nv,
-                                            &nt, s.patches);
+            hit = traverse_w8<false, PHONG>(s.wnodes, s.tris, xyz(a), xyz(b), a.w, b.w, st, t, tri, bu, bv, nv, nt,
+                                            s.patches);
         else if (any_hit)
-            hit = traverse<true, PHONG>(s.nodes, s.tris, xyz(a), xyz(b), a.w, b.w, stack, t, tri, bu, bv, &nv, &nt,
+            hit = traverse<true, PHONG>(s.nodes, s.tris, xyz(a), xyz(b), a.w, b.w, st, t, tri, bu, bv, nv, nt,
                                         s.patches);
         else
-            hit = traverse<false, PHONG>(s.nodes, s.tris, xyz(a), xyz(b), a.w, b.w, stack, t, tri, bu, bv, &nv, &nt,
+            hit = traverse<false, PHONG>(s.nodes, s.tris, xyz(a), xyz(b), a.w, b.w, st, t, tri, bu, bv, nv, nt,
                                          s.patches);
         uint32_t gid = MISS, pid = MISS;
         f3 ng = mk(0.f, 0.f, 0.f);
@@ -1159,36 +1161,56 @@ static WaveArgs make_args(const WaveBuffers &b, int parity, const RenderLaunch &
     return w;
 }
 
-// the traversal kernel instantiation for the scene: block size x (Phong patches) x (BVH width)
+// the traversal kernel instantiation for the scene: block size x (Phong patches) x (BVH width) x
+// (visit counters, for profiled renders)
 enum TraceLaunch { TRACE_EXTEND, TRACE_SHADOW, TRACE_SHADOW_PENDING, TRACE_PAIR };
 
-template <int BLOCK, bool PHONG, bool WIDE>
-void launch_trace_4(TraceLaunch what, const DevScene &s, const WaveArgs &w, const RenderLaunch &r, cudaStream_t st) {
+// bytes of the traversal stacks of a block; more than 48 KB (a 256-thread block on a tree deeper
+// than 46 levels) needs the kernel's consent
+template <class Kernel> size_t stack_bytes(Kernel *kernel, const DevScene &s, int block) {
+    const size_t bytes = size_t(s.stack_words) * size_t(block) * 4;
+    if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
+    return bytes;
+}
+
+template <int BLOCK, class Kernel, class... Args>
+void launch_stacked(Kernel *kernel, const DevScene &s, const WaveArgs &w, int grid, cudaStream_t st, Args... args) {
+    kernel<<<grid, BLOCK, stack_bytes(kernel, s, BLOCK), st>>>(s, w, args...);
+}
+
+template <int BLOCK, bool PHONG, bool WIDE, bool COUNT>
+void launch_trace_5(TraceLaunch what, const DevScene &s, const WaveArgs &w, int grid, cudaStream_t st) {
     switch (what) {
-        case TRACE_EXTEND: k_extend<BLOCK, PHONG, WIDE><<<r.grid_trace, BLOCK, 0, st>>>(s, w); break;
-        case TRACE_SHADOW: k_shadow<BLOCK, PHONG, WIDE><<<r.grid_trace, BLOCK, 0, st>>>(s, w, CTR_SHADOW); break;
+        case TRACE_EXTEND: launch_stacked<BLOCK>(k_extend<BLOCK, PHONG, WIDE, COUNT>, s, w, grid, st); break;
+        case TRACE_SHADOW: launch_stacked<BLOCK>(k_shadow<BLOCK, PHONG, WIDE, COUNT>, s, w, grid, st, int(CTR_SHADOW)); break;
         case TRACE_SHADOW_PENDING:
-            k_shadow<BLOCK, PHONG, WIDE><<<r.grid_trace, BLOCK, 0, st>>>(s, w, CTR_SHADOW_PENDING);
+            launch_stacked<BLOCK>(k_shadow<BLOCK, PHONG, WIDE, COUNT>, s, w, grid, st, int(CTR_SHADOW_PENDING));
             break;
         case TRACE_PAIR:
-            if (PHONG) k_trace_pair_phong<BLOCK, WIDE><<<r.grid_trace, BLOCK, 0, st>>>(s, w);
-            else k_trace_pair<BLOCK, WIDE><<<r.grid_trace, BLOCK, 0, st>>>(s, w);
+            if (PHONG) launch_stacked<BLOCK>(k_trace_pair_phong<BLOCK, WIDE, COUNT>, s, w, grid, st);
+            else launch_stacked<BLOCK>(k_trace_pair<BLOCK, WIDE, COUNT>, s, w, grid, st);
             break;
     }
 }
 
+template <int BLOCK, bool PHONG, bool WIDE>
+void launch_trace_4(TraceLaunch what, const DevScene &s, const WaveArgs &w, int grid, cudaStream_t st) {
+    if (w.prof) launch_trace_5<BLOCK, PHONG, WIDE, true>(what, s, w, grid, st);
+    else launch_trace_5<BLOCK, PHONG, WIDE, false>(what, s, w, grid, st);
+}
+
 template <int BLOCK>
-void launch_trace_3(TraceLaunch what, const DevScene &s, const WaveArgs &w, const RenderLaunch &r, cudaStream_t st) {
-    if (s.patches && s.wnodes) launch_trace_4<BLOCK, true, true>(what, s, w, r, st);
-    else if (s.patches) launch_trace_4<BLOCK, true, false>(what, s, w, r, st);
-    else if (s.wnodes) launch_trace_4<BLOCK, false, true>(what, s, w, r, st);
-    else launch_trace_4<BLOCK, false, false>(what, s, w, r, st);
+void launch_trace_3(TraceLaunch what, const DevScene &s, const WaveArgs &w, int grid, cudaStream_t st) {
+    if (s.patches && s.wnodes) launch_trace_4<BLOCK, true, true>(what, s, w, grid, st);
+    else if (s.patches) launch_trace_4<BLOCK, true, false>(what, s, w, grid, st);
+    else if (s.wnodes) launch_trace_4<BLOCK, false, true>(what, s, w, grid, st);
+    else launch_trace_4<BLOCK, false, false>(what, s, w, grid, st);
 }
 
 void launch_trace(TraceLaunch what, const DevScene &s, const WaveArgs &w, const RenderLaunch &r, cudaStream_t st) {
-    if (r.trace_block == 64) launch_trace_3<64>(what, s, w, r, st);
-    else if (r.trace_block == 256) launch_trace_3<256>(what, s, w, r, st);
-    else launch_trace_3<128>(what, s, w, r, st);
+    if (r.trace_block == 64) launch_trace_3<64>(what, s, w, r.grid_trace, st);
+    else if (r.trace_block == 256) launch_trace_3<256>(what, s, w, r.grid_trace, st);
+    else launch_trace_3<128>(what, s, w, r.grid_trace, st);
 }
 
 void launch_kernel(int which, const DevScene &s, const WaveBuffers &b, const RenderLaunch &r, int parity,
@@ -1259,10 +1281,11 @@ void launch_resolve(const double *film, double *out, const RenderLaunch &r, cuda
 
 void launch_trace_batch(const DevScene &s, const float4 *rays, uint32_t n, int any_hit, float4 *out, uint32_t *visits,
                         int grid, cudaStream_t st) {
-    if (s.patches && s.wnodes) k_trace_batch<true, true><<<grid, kTraceBlock, 0, st>>>(s, rays, n, any_hit, out, visits);
-    else if (s.patches) k_trace_batch<true, false><<<grid, kTraceBlock, 0, st>>>(s, rays, n, any_hit, out, visits);
-    else if (s.wnodes) k_trace_batch<false, true><<<grid, kTraceBlock, 0, st>>>(s, rays, n, any_hit, out, visits);
-    else k_trace_batch<false, false><<<grid, kTraceBlock, 0, st>>>(s, rays, n, any_hit, out, visits);
+    const size_t bytes = size_t(s.stack_words) * kTraceBlock * 4;   // at most 33 KB
+    if (s.patches && s.wnodes) k_trace_batch<true, true><<<grid, kTraceBlock, bytes, st>>>(s, rays, n, any_hit, out, visits);
+    else if (s.patches) k_trace_batch<true, false><<<grid, kTraceBlock, bytes, st>>>(s, rays, n, any_hit, out, visits);
+    else if (s.wnodes) k_trace_batch<false, true><<<grid, kTraceBlock, bytes, st>>>(s, rays, n, any_hit, out, visits);
+    else k_trace_batch<false, false><<<grid, kTraceBlock, bytes, st>>>(s, rays, n, any_hit, out, visits);
 }
 
 void launch_cdf_build(const double *weights, const uint32_t *offsets, uint32_t ntables, float *cdf, float *pdf,
@@ -1278,28 +1301,28 @@ void launch_scale_pdf(const double *weights, double total, float *pdf, size_t n,
     k_scale_pdf<<<592, 256, 0, st>>>(weights, total, pdf, n);
 }
 
-template <int BLOCK, bool PHONG, bool WIDE> int extend_occupancy() {
+template <int BLOCK, class Kernel> int resident_blocks(Kernel *kernel, const DevScene &s) {
     int nb = 0;
-    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_extend<BLOCK, PHONG, WIDE>, BLOCK, 0);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, BLOCK, stack_bytes(kernel, s, BLOCK));
     return nb;
 }
 
-template <int BLOCK> int extend_occupancy_3(bool phong, bool wide) {
-    if (phong && wide) return extend_occupancy<BLOCK, true, true>();
-    if (phong) return extend_occupancy<BLOCK, true, false>();
-    if (wide) return extend_occupancy<BLOCK, false, true>();
-    return extend_occupancy<BLOCK, false, false>();
+template <int BLOCK> int trace_occupancy_of(const DevScene &s) {
+    if (s.patches && s.wnodes) return resident_blocks<BLOCK>(k_trace_pair_phong<BLOCK, true, false>, s);
+    if (s.patches) return resident_blocks<BLOCK>(k_trace_pair_phong<BLOCK, false, false>, s);
+    if (s.wnodes) return resident_blocks<BLOCK>(k_trace_pair<BLOCK, true, false>, s);
+    return resident_blocks<BLOCK>(k_trace_pair<BLOCK, false, false>, s);
 }
 
-int occupancy_blocks(int which, int trace_block, bool phong, bool wide) {
+int trace_occupancy(const DevScene &s, int trace_block) {
+    if (trace_block == 64) return trace_occupancy_of<64>(s);
+    if (trace_block == 256) return trace_occupancy_of<256>(s);
+    return trace_occupancy_of<128>(s);
+}
+
+int shade_occupancy() {
     int nb = 0;
-    if (which == 0) {
-        if (trace_block == 64) nb = extend_occupancy_3<64>(phong, wide);
-        else if (trace_block == 256) nb = extend_occupancy_3<256>(phong, wide);
-        else nb = extend_occupancy_3<128>(phong, wide);
-    } else {
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_shade<false, false, false>, kShadeBlock, 0);
-    }
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_shade<false, false, false>, kShadeBlock, 0);
     return nb;
 }
 

@@ -196,8 +196,8 @@ extern "C" int wr_render_device_noalloc(wr_scene *scene, const wr_render_desc *d
     if (desc.max_iterations > 0) r.iter_limit = std::min(r.iter_limit, uint32_t(desc.max_iterations));
     r.trace_block = (desc.trace_block == 64 || desc.trace_block == 256) ? desc.trace_block : 128;
     r.grid_trace = desc.grid_trace > 0 ? desc.grid_trace
-                                       : sms * std::max(1, wrk::occupancy_blocks(0, r.trace_block, v.dev.patches != nullptr, v.dev.wnodes != nullptr));
-    r.grid_shade = desc.grid_shade > 0 ? desc.grid_shade : sms * (wrk::occupancy_blocks(1) > 0 ? wrk::occupancy_blocks(1) : 1);
+                                       : sms * std::max(1, wrk::trace_occupancy(v.dev, r.trace_block));
+    r.grid_shade = desc.grid_shade > 0 ? desc.grid_shade : sms * std::max(1, wrk::shade_occupancy());
     if (desc.fetch_threshold < 0 || desc.fetch_threshold > 32)
         return fail(WR_ERR_INVALID_ARGUMENT, "fetch_threshold must be 0..32");
     r.fetch_min = desc.fetch_threshold > 0 ? desc.fetch_threshold : 20;

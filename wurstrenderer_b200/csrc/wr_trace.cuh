@@ -5,10 +5,9 @@
 // * Binary BVH, both child boxes of a node in one 64-byte record fetched as two
 //   32-byte vector loads through the read-only path (ld.global.nc.v8.f32; four 16-byte
 //   loads measured 4.7 % slower on the 1M-triangle workload).
-// * Near-child-first descent; the far child is pushed on a per-ray stack whose
-//   first kSmemStack entries live in shared memory (one column per thread, so a
-//   warp's pushes hit 32 different banks) and whose rare deeper entries spill to
-//   a small local array. The builder bounds the tree depth by kMaxStack.
+// * Near-child-first descent; the far child is pushed on a per-ray stack that lies
+//   whole in shared memory (one column per thread, so a warp's pushes hit 32
+//   different banks), as deep as the scene's tree.
 // * Watertight ray/triangle test in FP32 (Woop, Benthin, Wald, "Watertight
 //   Ray/Triangle Intersection", JCGT 2013): per-ray shear to a frame where the
 //   ray is +z, 2-D edge functions evaluated without contraction so that the two
@@ -150,156 +149,81 @@ __device__ __forceinline__ f3 surface_normal(float4 a, float4 b, float4 c, float
     return normalize(cross(xyz(b) - xyz(a), xyz(c) - xyz(a)));
 }
 
+constexpr int kTraceDone = 0x7fffffff;   // traversal finished; also the entry at the bottom of the stack
+
+// Per-ray traversal stack in shared memory, DevScene::stack_words entries per thread: the tree's
+// depth bounds the pushes of a ray, and the bottom entry is kTraceDone, so neither push nor pop
+// checks a bound or branches. push_if and pop_if compile to predicated instructions that the whole
+// warp runs once. With 8 entries in shared memory and the rest in local memory a node visit of the
+// 1.16M-triangle frame ran its push with 4.4 lanes and its pop with 3.6, each on a shared and a
+// local path (127 warp-instructions per visit of a warp, 101 with this stack), and more of the
+// accesses went to local memory than to shared; that frame took 52.5 ms, 45.4 with this stack.
+// All entries in local memory measured 52.3 ms.
 struct TraceStack {
-    uint32_t *smem;   // kSmemStack x blockDim.x words, column = threadIdx.x
-    int stride;
-    int local[kMaxStack - kSmemStack];
-    int sp;
-    __device__ __forceinline__ void push(int v) {
-        if (sp < kSmemStack) smem[sp * stride] = uint32_t(v);
-        else local[sp - kSmemStack] = v;
-        ++sp;
+    uint32_t top;      // shared-space byte address of the next free entry of this thread's column
+    uint32_t bottom;   // the first entry above the sentinel
+    uint32_t stride;   // bytes between a thread's entries
+    __device__ __forceinline__ void init(uint32_t *column, uint32_t threads) {
+        column[0] = uint32_t(kTraceDone);
+        stride = 4u * threads;
+        bottom = uint32_t(__cvta_generic_to_shared(column)) + stride;
+        top = bottom;
     }
-    __device__ __forceinline__ int pop() {
-        --sp;
-        return sp < kSmemStack ? int(smem[sp * stride]) : local[sp - kSmemStack];
+    __device__ __forceinline__ void clear() { top = bottom; }
+    __device__ __forceinline__ bool empty() const { return top == bottom; }
+    __device__ __forceinline__ void push_if(bool p, int v) {
+        if (p) {
+            *static_cast<int *>(__cvta_shared_to_generic(top)) = v;
+            top += stride;
+        }
+    }
+    __device__ __forceinline__ void pop_if(bool p, int &v) {
+        if (p) {
+            top -= stride;
+            v = *static_cast<const int *>(__cvta_shared_to_generic(top));
+        }
     }
 };
 
-// Traverses the BVH. ANY_HIT: returns at the first accepted hit.
-// On return `t` holds the closest accepted distance; `tri` the leaf-order triangle (or MISS).
+// Traverses the BVH; resumable, for persistent kernels with dynamic ray fetching (Aila and Laine,
+// "Understanding the Efficiency of Ray Traversal on GPUs", HPG 2009, "replace terminated rays"): the
+// per-ray state (node, postponed leaf, stack, best hit) lives in the caller and survives between
+// calls. Returns true when this lane's ray is finished (any hit found for ANY_HIT, or the tree
+// exhausted); then `t` holds the closest accepted distance and `tri` the leaf-order triangle (or
+// MISS). UV: (bu, bv) receive a triangle hit's barycentrics too (a patch hit's normal always).
 //
-// Loop structure after Aila & Laine ("Understanding the Efficiency of Ray
-// Traversal on GPUs", HPG 2009): inner nodes and leaves are handled in two
-// separate loops, and a lane that reaches a leaf postpones it and keeps
-// descending inner nodes until every converged lane of the warp holds a leaf,
-// so that the triangle tests run with most lanes active. The warp vote only
-// steers scheduling; each lane's result does not depend on other lanes.
-template <bool ANY_HIT, bool PHONG = false>
-__device__ __forceinline__ bool traverse(const float4 *__restrict__ nodes, const float4 *__restrict__ tris, f3 o,
-                                         f3 d, float tmin, float tmax, uint32_t *smem_stack, float &t, uint32_t &tri,
-                                         float &bu, float &bv, uint32_t *node_visits = nullptr,
-                                         uint32_t *tri_tests = nullptr, const double *patches = nullptr) {
-    constexpr int kDone = 0x7fffffff;   // traversal finished (stack empty)
-    const RayPre r = ray_setup(o, d);
-    const PatchRay pr{o.x, o.y, o.z, d.x, d.y, d.z};
-    TraceStack st;
-    st.smem = smem_stack + threadIdx.x;
-    st.stride = blockDim.x;
-    st.sp = 0;
-    tri = MISS;
-    t = tmax;
-    int node = 0;    // next inner node (>= 0), a leaf code (< 0) or kDone
-    int leaf = 0;    // postponed leaf code (< 0), 0 when none
-    uint32_t nv = 0, nt = 0;
-    while (node != kDone) {
-        while (node >= 0 && node != kDone) {
-            float4 n0, n1, n2, n3;
-            ld_node(nodes + 4 * node, n0, n1, n2, n3);
-            ++nv;
-            const float e0 = box_entry(r, n0.x, n0.y, n0.z, n0.w, n2.x, n2.y, tmin, t);
-            const float e1 = box_entry(r, n1.x, n1.y, n1.z, n1.w, n2.z, n2.w, tmin, t);
-            const int c0 = __float_as_int(n3.x), c1 = __float_as_int(n3.y);
-            const bool h0 = e0 != __int_as_float(0x7f800000), h1 = e1 != __int_as_float(0x7f800000);
-            if (h0 && h1) {
-                int near = c0, far = c1;
-                if (e1 < e0) { near = c1; far = c0; }
-                st.push(far);
-                node = near;
-            } else if (h0) {
-                node = c0;
-            } else if (h1) {
-                node = c1;
-            } else {
-                node = st.sp ? st.pop() : kDone;
-            }
-            if (node < 0 && leaf == 0) {   // postpone the first leaf found, keep descending
-                leaf = node;
-                node = st.sp ? st.pop() : kDone;
-            }
-            if (!__any_sync(__activemask(), leaf == 0)) break;
-        }
-        while (leaf < 0) {
-            const uint32_t code = uint32_t(leaf);
-            const uint32_t first = code & 0x07ffffffu;
-            const uint32_t count = ((code >> 27) & 0xfu) + 1u;
-            for (uint32_t i = first; i < first + count; ++i) {
-                const float4 a = __ldg(tris + 3 * i + 0);
-                const float4 b = __ldg(tris + 3 * i + 1);
-                const float4 c = __ldg(tris + 3 * i + 2);
-                ++nt;
-                if (PHONG && (__float_as_uint(a.w) & wrp::kPatchFlag)) {
-                    if (patch_leaf_test(r, pr, patches, i, a, b, c, tmin, t, bu, bv)) {
-                        tri = i;
-                        if (ANY_HIT) {
-                            if (node_visits) { *node_visits += nv; *tri_tests += nt; }
-                            return true;
-                        }
-                    }
-                    continue;
-                }
-                float th, uh, vh;
-                if (tri_test(r, a, b, c, tmin, t, th, uh, vh)) {
-                    if (ANY_HIT) {
-                        t = th; tri = i; bu = uh; bv = vh;
-                        if (node_visits) { *node_visits += nv; *tri_tests += nt; }
-                        return true;
-                    }
-                    if (th < t || tri == MISS) { t = th; tri = i; bu = uh; bv = vh; }
-                }
-            }
-            leaf = 0;
-            if (node < 0 && node != kDone) {   // the traversal is sitting on another leaf
-                leaf = node;
-                node = st.sp ? st.pop() : kDone;
-            }
-        }
-    }
-    if (node_visits) { *node_visits += nv; *tri_tests += nt; }
-    return tri != MISS;
-}
+// Inner nodes and leaves are handled in two separate loops (while-while, the same paper): a lane
+// that reaches a leaf postpones it and keeps descending inner nodes until fewer than kLeafWait lanes
+// of the warp still look for one, so that the triangle tests run with most lanes active; after each
+// leaf pass the warp returns when fewer than `min_active` of its lanes are still traversing, so that
+// the caller can hand new rays to the finished ones. The votes only steer the schedule; each lane's
+// result does not depend on other lanes. kLeafWait = 1 / 4 / 8 / 12 measured 45.3 / 43.8 / 44.0 /
+// 44.7 ms for the 1.16M-triangle frame.
+constexpr int kLeafWait = 4;
 
-// Resumable form of `traverse` for persistent kernels with dynamic ray fetching (Aila &
-// Laine 2009, "replace terminated rays"): the per-ray state (node, postponed leaf, stack,
-// best hit) lives in the caller and survives between calls. The while-while loop runs as in
-// `traverse`, but after each leaf pass the warp leaves it when fewer than `min_active` of its
-// lanes are still traversing, so that the caller can hand new rays to the finished lanes.
-// Returns true when this lane's ray is finished (any hit found for ANY_HIT, or the tree
-// exhausted); the result is the same as `traverse`'s, only the schedule differs.
-constexpr int kTraceDone = 0x7fffffff;
-
-template <bool ANY_HIT, bool PHONG = false>
+template <bool ANY_HIT, bool PHONG, bool UV, bool COUNT>
 __device__ __forceinline__ bool traverse_steps(const float4 *__restrict__ nodes, const float4 *__restrict__ tris,
                                                const RayPre &r, float tmin, float &t, uint32_t &tri, float &bu,
                                                float &bv, int &node, int &leaf, TraceStack &st, uint32_t &nv,
                                                uint32_t &nt, int min_active, const double *patches = nullptr,
                                                const PatchRay &pr = PatchRay{}) {
     while (node != kTraceDone) {
-        while (node >= 0 && node != kTraceDone) {
+        while (uint32_t(node) < uint32_t(kTraceDone)) {   // an inner node
             float4 n0, n1, n2, n3;
             ld_node(nodes + 4 * node, n0, n1, n2, n3);
-            ++nv;
+            if (COUNT) ++nv;
             const float e0 = box_entry(r, n0.x, n0.y, n0.z, n0.w, n2.x, n2.y, tmin, t);
             const float e1 = box_entry(r, n1.x, n1.y, n1.z, n1.w, n2.z, n2.w, tmin, t);
             const int c0 = __float_as_int(n3.x), c1 = __float_as_int(n3.y);
             const bool h0 = e0 != __int_as_float(0x7f800000), h1 = e1 != __int_as_float(0x7f800000);
-            if (h0 && h1) {
-                int near = c0, far = c1;
-                if (e1 < e0) { near = c1; far = c0; }
-                st.push(far);
-                node = near;
-            } else if (h0) {
-                node = c0;
-            } else if (h1) {
-                node = c1;
-            } else {
-                node = st.sp ? st.pop() : kTraceDone;
-            }
-            if (node < 0 && leaf == 0) {   // postpone the first leaf found, keep descending
-                leaf = node;
-                node = st.sp ? st.pop() : kTraceDone;
-            }
-            if (!__any_sync(__activemask(), leaf == 0)) break;
+            const bool swap = e1 < e0;   // a missed child's entry is +inf
+            st.push_if(h0 && h1, swap ? c0 : c1);
+            node = swap ? c1 : c0;
+            st.pop_if(!h0 && !h1, node);
+            const bool take = node < 0 && leaf == 0;   // postpone the first leaf found, keep descending
+            leaf = take ? node : leaf;
+            st.pop_if(take, node);
+            if (__popc(__ballot_sync(__activemask(), leaf == 0)) < kLeafWait) break;
         }
         while (leaf < 0) {
             const uint32_t code = uint32_t(leaf);
@@ -309,7 +233,7 @@ __device__ __forceinline__ bool traverse_steps(const float4 *__restrict__ nodes,
                 const float4 a = __ldg(tris + 3 * i + 0);
                 const float4 b = __ldg(tris + 3 * i + 1);
                 const float4 c = __ldg(tris + 3 * i + 2);
-                ++nt;
+                if (COUNT) ++nt;
                 if (PHONG && (__float_as_uint(a.w) & wrp::kPatchFlag)) {
                     if (patch_leaf_test(r, pr, patches, i, a, b, c, tmin, t, bu, bv)) {
                         tri = i;
@@ -323,24 +247,43 @@ __device__ __forceinline__ bool traverse_steps(const float4 *__restrict__ nodes,
                 }
                 float th, uh, vh;
                 if (tri_test(r, a, b, c, tmin, t, th, uh, vh)) {
+                    if (ANY_HIT || th < t || tri == MISS) {
+                        t = th;
+                        tri = i;
+                        if (UV || PHONG) { bu = uh; bv = vh; }
+                    }
                     if (ANY_HIT) {
-                        t = th; tri = i; bu = uh; bv = vh;
                         node = kTraceDone;
                         leaf = 0;
                         return true;
                     }
-                    if (th < t || tri == MISS) { t = th; tri = i; bu = uh; bv = vh; }
                 }
             }
             leaf = 0;
-            if (node < 0 && node != kTraceDone) {   // the traversal is sitting on another leaf
+            if (node < 0) {   // the traversal is sitting on another leaf
                 leaf = node;
-                node = st.sp ? st.pop() : kTraceDone;
+                st.pop_if(true, node);
             }
         }
         if (node != kTraceDone && __popc(__activemask()) < min_active) return false;
     }
     return true;
+}
+
+// one whole query (the k_trace_batch path)
+template <bool ANY_HIT, bool PHONG>
+__device__ __forceinline__ bool traverse(const float4 *__restrict__ nodes, const float4 *__restrict__ tris, f3 o,
+                                         f3 d, float tmin, float tmax, TraceStack &st, float &t, uint32_t &tri,
+                                         float &bu, float &bv, uint32_t &nv, uint32_t &nt, const double *patches) {
+    const RayPre r = ray_setup(o, d);
+    const PatchRay pr{o.x, o.y, o.z, d.x, d.y, d.z};
+    int node = 0, leaf = 0;
+    tri = MISS;
+    t = tmax;
+    st.clear();
+    traverse_steps<ANY_HIT, PHONG, true, true>(nodes, tris, r, tmin, t, tri, bu, bv, node, leaf, st, nv, nt, 0, patches,
+                                               pr);
+    return tri != MISS;
 }
 
 // ------------------------------------------------------------------------
@@ -367,7 +310,7 @@ __device__ __forceinline__ float wq_byte(uint32_t lo, uint32_t hi, int k) {
     return __uint_as_float(__byte_perm(k < 4 ? lo : hi, 0x4B000000u, 0x7540u | uint32_t(k & 3))) - 8388608.0f;
 }
 
-template <bool ANY_HIT, bool PHONG = false>
+template <bool ANY_HIT, bool PHONG, bool UV, bool COUNT>
 __device__ __forceinline__ bool traverse_steps_w8(const uint4 *__restrict__ wnodes, const float4 *__restrict__ tris,
                                                   const RayPre &r, uint32_t oct, float tmin, float &t, uint32_t &tri,
                                                   float &bu, float &bv, WideState &ws, TraceStack &st, uint32_t &nv,
@@ -381,7 +324,7 @@ __device__ __forceinline__ bool traverse_steps_w8(const uint4 *__restrict__ wnod
             const uint4 n2 = __ldg(wnodes + 5 * ws.node + 2);
             const uint4 n3 = __ldg(wnodes + 5 * ws.node + 3);
             const uint4 n4 = __ldg(wnodes + 5 * ws.node + 4);
-            ++nv;
+            if (COUNT) ++nv;
             const float sx = __uint_as_float((n0.w & 0xffu) << 23) * r.ix;
             const float sy = __uint_as_float(((n0.w >> 8) & 0xffu) << 23) * r.iy;
             const float sz = __uint_as_float(((n0.w >> 16) & 0xffu) << 23) * r.iz;
@@ -425,14 +368,14 @@ __device__ __forceinline__ bool traverse_steps_w8(const uint4 *__restrict__ wnod
                 const float4 a = __ldg(tris + 3 * i + 0);
                 const float4 b = __ldg(tris + 3 * i + 1);
                 const float4 c = __ldg(tris + 3 * i + 2);
-                ++nt;
+                if (COUNT) ++nt;
                 if (PHONG && (__float_as_uint(a.w) & wrp::kPatchFlag)) {
                     if (patch_leaf_test(r, pr, patches, i, a, b, c, tmin, t, bu, bv)) {
                         tri = i;
                         if (ANY_HIT) {
                             ws.node = -1;
                             ws.grp = 0;
-                            st.sp = 0;
+                            st.clear();
                             return true;
                         }
                     }
@@ -440,18 +383,21 @@ __device__ __forceinline__ bool traverse_steps_w8(const uint4 *__restrict__ wnod
                 }
                 float th, uh, vh;
                 if (tri_test(r, a, b, c, tmin, t, th, uh, vh)) {
+                    if (ANY_HIT || th < t || tri == MISS) {
+                        t = th;
+                        tri = i;
+                        if (UV || PHONG) { bu = uh; bv = vh; }
+                    }
                     if (ANY_HIT) {
-                        t = th; tri = i; bu = uh; bv = vh;
                         ws.node = -1;
                         ws.grp = 0;
-                        st.sp = 0;
+                        st.clear();
                         return true;
                     }
-                    if (th < t || tri == MISS) { t = th; tri = i; bu = uh; bv = vh; }
                 }
             }
             if (inner) {
-                if (ws.grp & 0xffu) st.push(int(ws.grp));
+                st.push_if((ws.grp & 0xffu) != 0u, int(ws.grp));
                 ws.grp = uint32_t(ws.node) << 8 | inner;
                 ws.gbase = n1.x;
                 ws.gimask = imask;
@@ -460,8 +406,10 @@ __device__ __forceinline__ bool traverse_steps_w8(const uint4 *__restrict__ wnod
         }
         // next child: the lowest hit position of the current group, else a popped group
         if (!(ws.grp & 0xffu)) {
-            if (!st.sp) return true;
-            ws.grp = uint32_t(st.pop());
+            if (st.empty()) return true;
+            int grp;
+            st.pop_if(true, grp);
+            ws.grp = uint32_t(grp);
             const uint32_t pn = ws.grp >> 8;
             const uint32_t *pw = reinterpret_cast<const uint32_t *>(wnodes + 5 * pn);
             ws.gbase = __ldg(pw + 4);
@@ -480,24 +428,18 @@ __device__ __forceinline__ uint32_t ray_octant(f3 d) {
 }
 
 // one whole query on the compressed 8-wide BVH (the k_trace_batch path)
-template <bool ANY_HIT, bool PHONG = false>
+template <bool ANY_HIT, bool PHONG>
 __device__ __forceinline__ bool traverse_w8(const uint4 *__restrict__ wnodes, const float4 *__restrict__ tris, f3 o,
-                                            f3 d, float tmin, float tmax, uint32_t *smem_stack, float &t,
-                                            uint32_t &tri, float &bu, float &bv, uint32_t *node_visits = nullptr,
-                                            uint32_t *tri_tests = nullptr, const double *patches = nullptr) {
+                                            f3 d, float tmin, float tmax, TraceStack &st, float &t, uint32_t &tri,
+                                            float &bu, float &bv, uint32_t &nv, uint32_t &nt, const double *patches) {
     const RayPre r = ray_setup(o, d);
     const PatchRay pr{o.x, o.y, o.z, d.x, d.y, d.z};
-    TraceStack st;
-    st.smem = smem_stack + threadIdx.x;
-    st.stride = blockDim.x;
-    st.sp = 0;
     WideState ws{0, 0u, 0u, 0u};
     tri = MISS;
     t = tmax;
-    uint32_t nv = 0, nt = 0;
-    traverse_steps_w8<ANY_HIT, PHONG>(wnodes, tris, r, ray_octant(d), tmin, t, tri, bu, bv, ws, st, nv, nt, 0,
-                                      patches, pr);
-    if (node_visits) { *node_visits += nv; *tri_tests += nt; }
+    st.clear();
+    traverse_steps_w8<ANY_HIT, PHONG, true, true>(wnodes, tris, r, ray_octant(d), tmin, t, tri, bu, bv, ws, st, nv, nt,
+                                                  0, patches, pr);
     return tri != MISS;
 }
 
