@@ -29,7 +29,7 @@ _lib = None
 def build(with_reference: bool = True) -> None:
     """Compiles the oracle (and the reference harness when the reference is present)."""
     subprocess.run(["make", "-s", "-C", HERE, "liboracle_nee.so"], check=True)
-    if with_reference and os.path.isdir(REFERENCE_ROOT):
+    if with_reference and os.path.isdir(os.path.join(REFERENCE_ROOT, "src")):
         subprocess.run(["make", "-s", "-C", HERE, "-j8", "ref", "REF=" + REFERENCE_ROOT], check=True)
 
 
