@@ -303,3 +303,20 @@ def test_scene_without_any_emitter_renders_black(wr_lib, tmp_path, integrator):
         assert sc.info["num_lights"] == 0 and sc.info["has_envmap"] == 0
         img = sc.render(spp=16, seed=3, integrator=integrator)
     assert img.shape == (16, 24, 3) and np.isfinite(img).all() and not img.any()
+
+
+@pytest.mark.parametrize("integrator", ["nextevent_path_tracer", "primitive_path_tracer", "light_splatting"])
+@pytest.mark.parametrize("nverts", [1, 2, 3, 10, 64, 65])
+def test_one_wave_renders_match_graphs(wr_lib, nverts, integrator):
+    """A render whose samples fit the wavefront is launched without a graph, for exactly the bounce
+    iterations that its paths can have; the same samples through a smaller wavefront are one graph."""
+    path, _ = golden_scene("cornell")
+    kw = dict(spp=3, num_path_vertices=nverts, seed=4, integrator=integrator)
+    with wr_lib.Scene.from_file(path) as sc:
+        chained = sc.render(**kw)
+        if nverts > 1:
+            assert sc.stats["iterations"] == (nverts if nverts <= 64 else sc.stats["iterations"])
+        graph = sc.render(queue_capacity=1024, **kw)
+        profiled = sc.render(profile=3, **kw)
+    assert np.allclose(chained, graph, rtol=1e-9, atol=1e-12)
+    assert np.allclose(chained, profiled, rtol=1e-9, atol=1e-12)

@@ -339,6 +339,15 @@ __device__ __forceinline__ uint32_t job_seed(const DevJob &J, uint32_t job) { re
 
 __device__ __forceinline__ uint32_t lane_id() { return threadIdx.x & 31u; }
 
+// First statement of every kernel of the bounce loop. Where it was launched with programmatic
+// stream serialization (a render without a graph), its blocks may be set up while the kernel before
+// it still runs, and wait here until that kernel is complete and its writes are visible; launched in
+// any other way, both instructions do nothing.
+__device__ __forceinline__ void chain_begin() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
 // warp-aggregated append: one atomic per warp, lane offsets from ballot/popc
 __device__ __forceinline__ uint32_t warp_append(uint32_t *counter, bool pred, uint32_t &total_out) {
     const uint32_t mask = __ballot_sync(0xffffffffu, pred);
@@ -464,6 +473,7 @@ __device__ __forceinline__ void trace_queue(const DevScene &s, const WaveArgs &w
 // dynamic shared memory of the traversal kernels: DevScene::stack_words x BLOCK words
 template <int BLOCK, bool PHONG, bool WIDE, bool COUNT>
 __global__ void __launch_bounds__(BLOCK) k_extend(DevScene s, WaveArgs w) {
+    chain_begin();
     extern __shared__ uint32_t stack[];
     trace_queue<BLOCK, false, PHONG, WIDE, COUNT>(s, w, stack, CTR_ACTIVE);
 }
@@ -774,6 +784,7 @@ __device__ __forceinline__ void shade_path(const DevScene &s, const WaveArgs &w,
 // blocks (64 registers) gained nothing on it and cost 0.7 % on the plain 1M-triangle render.
 template <bool GUIDED, bool NEE_ONLY, bool RECORD>
 __global__ void __launch_bounds__(kShadeBlock, 3) k_shade(DevScene s, WaveArgs w) {
+    chain_begin();
     const uint32_t n = w.ctr[CTR_ACTIVE];
     if (w.prof && blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(w.prof + 1, (unsigned long long)n);
     const uint32_t warp_global = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -826,6 +837,7 @@ __device__ __forceinline__ uint32_t tile_order_pixel(uint32_t q, uint32_t W, uin
 }
 
 __global__ void __launch_bounds__(kShadeBlock) k_raygen(DevScene s, WaveArgs w) {
+    chain_begin();
     const uint32_t filled = w.ctr[CTR_NEXT];
     const unsigned long long issued = *w.sample_next;
     const uint32_t n_new = new_samples(w, filled, issued);
@@ -941,6 +953,7 @@ __global__ void __launch_bounds__(kShadeBlock) k_raygen(DevScene s, WaveArgs w) 
 
 template <int BLOCK, bool PHONG, bool WIDE, bool COUNT>
 __global__ void __launch_bounds__(BLOCK) k_shadow(DevScene s, WaveArgs w, int count_ctr) {
+    chain_begin();
     extern __shared__ uint32_t stack[];
     trace_queue<BLOCK, true, PHONG, WIDE, COUNT>(s, w, stack, count_ctr);
 }
@@ -953,6 +966,7 @@ __global__ void __launch_bounds__(BLOCK) k_shadow(DevScene s, WaveArgs w, int co
 // shade appends to the shadow queue only after this launch).
 template <int BLOCK, bool PHONG, bool WIDE, bool COUNT>
 __device__ __forceinline__ void trace_pair(const DevScene &s, const WaveArgs &w) {
+    chain_begin();
     extern __shared__ uint32_t stack[];
     trace_queue<BLOCK, false, PHONG, WIDE, COUNT>(s, w, stack, CTR_ACTIVE);
     trace_queue<BLOCK, true, PHONG, WIDE, COUNT>(s, w, stack, CTR_SHADOW_PENDING);
@@ -972,6 +986,7 @@ __global__ void __launch_bounds__(BLOCK, (384 / BLOCK > 0 ? 384 / BLOCK : 1)) k_
 
 // queue bookkeeping between iterations (one thread); also drives the graph's while loop
 __global__ void k_advance(WaveArgs w) {
+    chain_begin();
     const uint32_t filled = w.ctr[CTR_NEXT];
     const unsigned long long issued = *w.sample_next;
     const uint32_t n_new = new_samples(w, filled, issued);
@@ -998,6 +1013,7 @@ __global__ void k_advance(WaveArgs w) {
 // final image = base / spp + splat / (spp * W * H) per job (film.h:70-90)
 __global__ void k_resolve(const double *film, double *out, uint32_t total_pix, const DevJob *jobs, int njobs,
                           DevJob job0) {
+    chain_begin();
     for (size_t i = blockIdx.x * size_t(blockDim.x) + threadIdx.x; i < 3 * size_t(total_pix);
          i += size_t(gridDim.x) * blockDim.x) {
         const uint32_t pix = uint32_t(i / 3);
@@ -1161,6 +1177,22 @@ static WaveArgs make_args(const WaveBuffers &b, int parity, const RenderLaunch &
     return w;
 }
 
+// launches a kernel of the bounce loop; `chain`: its set-up may overlap the kernel before it (chain_begin)
+template <class... Params, class... Args>
+void launch_chained(void (*kernel)(Params...), int grid, int block, size_t smem, cudaStream_t st, bool chain, Args... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(unsigned(grid));
+    cfg.blockDim = dim3(unsigned(block));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = chain ? 1 : 0;
+    cudaLaunchKernelEx(&cfg, kernel, args...);   // an error stays for the caller's cudaGetLastError
+}
+
 // the traversal kernel instantiation for the scene: block size x (Phong patches) x (BVH width) x
 // (visit counters, for profiled renders)
 enum TraceLaunch { TRACE_EXTEND, TRACE_SHADOW, TRACE_SHADOW_PENDING, TRACE_PAIR };
@@ -1174,43 +1206,44 @@ template <class Kernel> size_t stack_bytes(Kernel *kernel, const DevScene &s, in
 }
 
 template <int BLOCK, class Kernel, class... Args>
-void launch_stacked(Kernel *kernel, const DevScene &s, const WaveArgs &w, int grid, cudaStream_t st, Args... args) {
-    kernel<<<grid, BLOCK, stack_bytes(kernel, s, BLOCK), st>>>(s, w, args...);
+void launch_stacked(Kernel *kernel, const DevScene &s, const WaveArgs &w, const RenderLaunch &r, cudaStream_t st,
+                    Args... args) {
+    launch_chained(kernel, r.grid_trace, BLOCK, stack_bytes(kernel, s, BLOCK), st, r.chain != 0, s, w, args...);
 }
 
 template <int BLOCK, bool PHONG, bool WIDE, bool COUNT>
-void launch_trace_5(TraceLaunch what, const DevScene &s, const WaveArgs &w, int grid, cudaStream_t st) {
+void launch_trace_5(TraceLaunch what, const DevScene &s, const WaveArgs &w, const RenderLaunch &r, cudaStream_t st) {
     switch (what) {
-        case TRACE_EXTEND: launch_stacked<BLOCK>(k_extend<BLOCK, PHONG, WIDE, COUNT>, s, w, grid, st); break;
-        case TRACE_SHADOW: launch_stacked<BLOCK>(k_shadow<BLOCK, PHONG, WIDE, COUNT>, s, w, grid, st, int(CTR_SHADOW)); break;
+        case TRACE_EXTEND: launch_stacked<BLOCK>(k_extend<BLOCK, PHONG, WIDE, COUNT>, s, w, r, st); break;
+        case TRACE_SHADOW: launch_stacked<BLOCK>(k_shadow<BLOCK, PHONG, WIDE, COUNT>, s, w, r, st, int(CTR_SHADOW)); break;
         case TRACE_SHADOW_PENDING:
-            launch_stacked<BLOCK>(k_shadow<BLOCK, PHONG, WIDE, COUNT>, s, w, grid, st, int(CTR_SHADOW_PENDING));
+            launch_stacked<BLOCK>(k_shadow<BLOCK, PHONG, WIDE, COUNT>, s, w, r, st, int(CTR_SHADOW_PENDING));
             break;
         case TRACE_PAIR:
-            if (PHONG) launch_stacked<BLOCK>(k_trace_pair_phong<BLOCK, WIDE, COUNT>, s, w, grid, st);
-            else launch_stacked<BLOCK>(k_trace_pair<BLOCK, WIDE, COUNT>, s, w, grid, st);
+            if (PHONG) launch_stacked<BLOCK>(k_trace_pair_phong<BLOCK, WIDE, COUNT>, s, w, r, st);
+            else launch_stacked<BLOCK>(k_trace_pair<BLOCK, WIDE, COUNT>, s, w, r, st);
             break;
     }
 }
 
 template <int BLOCK, bool PHONG, bool WIDE>
-void launch_trace_4(TraceLaunch what, const DevScene &s, const WaveArgs &w, int grid, cudaStream_t st) {
-    if (w.prof) launch_trace_5<BLOCK, PHONG, WIDE, true>(what, s, w, grid, st);
-    else launch_trace_5<BLOCK, PHONG, WIDE, false>(what, s, w, grid, st);
+void launch_trace_4(TraceLaunch what, const DevScene &s, const WaveArgs &w, const RenderLaunch &r, cudaStream_t st) {
+    if (w.prof) launch_trace_5<BLOCK, PHONG, WIDE, true>(what, s, w, r, st);
+    else launch_trace_5<BLOCK, PHONG, WIDE, false>(what, s, w, r, st);
 }
 
 template <int BLOCK>
-void launch_trace_3(TraceLaunch what, const DevScene &s, const WaveArgs &w, int grid, cudaStream_t st) {
-    if (s.patches && s.wnodes) launch_trace_4<BLOCK, true, true>(what, s, w, grid, st);
-    else if (s.patches) launch_trace_4<BLOCK, true, false>(what, s, w, grid, st);
-    else if (s.wnodes) launch_trace_4<BLOCK, false, true>(what, s, w, grid, st);
-    else launch_trace_4<BLOCK, false, false>(what, s, w, grid, st);
+void launch_trace_3(TraceLaunch what, const DevScene &s, const WaveArgs &w, const RenderLaunch &r, cudaStream_t st) {
+    if (s.patches && s.wnodes) launch_trace_4<BLOCK, true, true>(what, s, w, r, st);
+    else if (s.patches) launch_trace_4<BLOCK, true, false>(what, s, w, r, st);
+    else if (s.wnodes) launch_trace_4<BLOCK, false, true>(what, s, w, r, st);
+    else launch_trace_4<BLOCK, false, false>(what, s, w, r, st);
 }
 
 void launch_trace(TraceLaunch what, const DevScene &s, const WaveArgs &w, const RenderLaunch &r, cudaStream_t st) {
-    if (r.trace_block == 64) launch_trace_3<64>(what, s, w, r.grid_trace, st);
-    else if (r.trace_block == 256) launch_trace_3<256>(what, s, w, r.grid_trace, st);
-    else launch_trace_3<128>(what, s, w, r.grid_trace, st);
+    if (r.trace_block == 64) launch_trace_3<64>(what, s, w, r, st);
+    else if (r.trace_block == 256) launch_trace_3<256>(what, s, w, r, st);
+    else launch_trace_3<128>(what, s, w, r, st);
 }
 
 void launch_kernel(int which, const DevScene &s, const WaveBuffers &b, const RenderLaunch &r, int parity,
@@ -1218,23 +1251,26 @@ void launch_kernel(int which, const DevScene &s, const WaveBuffers &b, const Ren
     const WaveArgs w = make_args(b, parity, r);
     switch (which) {
         case KERNEL_EXTEND: launch_trace(TRACE_EXTEND, s, w, r, st); break;
-        case KERNEL_SHADE:
-            if (w.lobes && w.records) k_shade<true, true, true><<<r.grid_shade, kShadeBlock, 0, st>>>(s, w);
-            else if (w.lobes) k_shade<true, true, false><<<r.grid_shade, kShadeBlock, 0, st>>>(s, w);
-            else if (w.records) k_shade<false, false, true><<<r.grid_shade, kShadeBlock, 0, st>>>(s, w);
-            else if (r.nee_only) k_shade<false, true, false><<<r.grid_shade, kShadeBlock, 0, st>>>(s, w);
-            else k_shade<false, false, false><<<r.grid_shade, kShadeBlock, 0, st>>>(s, w);
+        case KERNEL_SHADE: {
+            auto *kernel = k_shade<false, false, false>;
+            if (w.lobes && w.records) kernel = k_shade<true, true, true>;
+            else if (w.lobes) kernel = k_shade<true, true, false>;
+            else if (w.records) kernel = k_shade<false, false, true>;
+            else if (r.nee_only) kernel = k_shade<false, true, false>;
+            // after the inference kernel, which is not part of the chain, the launch waits as usual
+            launch_chained(kernel, r.grid_shade, kShadeBlock, 0, st, r.chain && !w.lobes, s, w);
             break;
+        }
         case KERNEL_GUIDE:
             if (r.guide)
                 wrg::guide_infer_wavefront(*r.guide, w.cur.o, w.cur.d, w.hit, w.ctr + CTR_ACTIVE, s.tris, s.tri_mat,
                                            b.lobes, b.capacity, r.guide_sms, st);
             break;
-        case KERNEL_RAYGEN: k_raygen<<<r.grid_shade, kShadeBlock, 0, st>>>(s, w); break;
+        case KERNEL_RAYGEN: launch_chained(k_raygen, r.grid_shade, kShadeBlock, 0, st, r.chain != 0, s, w); break;
         case KERNEL_SHADOW: launch_trace(TRACE_SHADOW, s, w, r, st); break;
         case KERNEL_TRACE_PAIR: launch_trace(TRACE_PAIR, s, w, r, st); break;
         case KERNEL_SHADOW_FLUSH: launch_trace(TRACE_SHADOW_PENDING, s, w, r, st); break;
-        case KERNEL_ADVANCE: k_advance<<<1, 1, 0, st>>>(w); break;
+        case KERNEL_ADVANCE: launch_chained(k_advance, 1, 1, 0, st, r.chain != 0, w); break;
         default: break;
     }
 }
@@ -1276,7 +1312,7 @@ void launch_prime(const DevScene &s, const WaveBuffers &b, const RenderLaunch &r
 }
 
 void launch_resolve(const double *film, double *out, const RenderLaunch &r, cudaStream_t st) {
-    k_resolve<<<592, 256, 0, st>>>(film, out, r.total_pix, r.jobs, r.num_jobs, r.job0);
+    launch_chained(k_resolve, 592, 256, 0, st, r.chain != 0, film, out, r.total_pix, r.jobs, r.num_jobs, r.job0);
 }
 
 void launch_trace_batch(const DevScene &s, const float4 *rays, uint32_t n, int any_hit, float4 *out, uint32_t *visits,

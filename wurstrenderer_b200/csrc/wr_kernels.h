@@ -43,6 +43,7 @@ struct RenderLaunch {
     int record;                 // 1: collect training records
     int guide_sms;              // SM count (grid of the inference kernel)
     int fetch_min;              // dynamic ray fetching threshold (lanes still traversing)
+    int chain;                  // 1: each kernel's set-up may overlap the kernel before it in the stream
     int nee_only;               // 1: every job is nextevent_path_tracer (shade without the other
                                 // integrators' branches); 0: any mix of integrators
 };
