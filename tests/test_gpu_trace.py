@@ -297,3 +297,22 @@ def test_deep_trees_and_the_stack(wr_lib, tmp_path, n, ratio, builder):
     assert np.array_equal(occ != 0, hits[0] >= 0)
     for im in images[1:]:
         assert np.allclose(im, images[0], rtol=1e-9, atol=1e-12)
+
+
+@pytest.mark.parametrize("name", ["hf", "phong"])
+@pytest.mark.parametrize("n", [1, 129, (1 << 20) - 1, 1 << 20, (1 << 20) + 5, (1 << 21) + 1])
+def test_long_batches_answer_like_short_ones(wr_lib, name, n):
+    """Batches around the length that the library sends to the device at a time: every ray's answers
+    are those of the fixture's own batch, whatever its place."""
+    path, _ = golden_scene(name)
+    rays = np.load("%s/%s_rays.npy" % (GOLDEN, name))
+    k = len(rays)
+    if name == "phong" and n > 1 << 20:
+        k = 300                      # the FP64 patch test on few distinct rays
+        rays = rays[:k]
+    take = np.arange(n) % k
+    with wr_lib.Scene.from_file(path) as sc:
+        few = sc.trace_closest(rays) + sc.trace_hits(rays)[3:] + (sc.trace_occluded(rays),)
+        many = sc.trace_closest(rays[take]) + sc.trace_hits(rays[take])[3:] + (sc.trace_occluded(rays[take]),)
+    for a, b in zip(few, many):
+        assert np.array_equal(a[take], b)

@@ -16,6 +16,7 @@
 #include <cmath>
 #include <cstring>
 #include <memory>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -95,6 +96,8 @@ struct wr_scene {
     int guide_step = 0;
     float box_lo[3] = {0.f, 0.f, 0.f}, box_inv[3] = {1.f, 1.f, 1.f};
     DevBuf w_rec[2], w_lobes, w_records, w_rec_count, g_scratch, g_scratch2, g_loss;
+    DevBuf q_rays, q_answers;   // ray batches: one chunk of rays and its answers
+    std::mutex ray_mutex;       // one batch at a time uses them
     uint32_t w_guide_capacity = 0, w_record_capacity = 0;
     uint32_t w_capacity = 0;
     size_t w_npix = 0;
@@ -1125,32 +1128,60 @@ void render_batch(wr_scene &s, const wr_job *jobs, int n, const wr_render_desc *
     render_jobs(s, hj, desc, out, on_host);
 }
 
-wrd::DevScene scene_for_queries(wr_scene &s) { return s.dev; }
+// One ray batch: the rays go to the device and the wanted answers come back into the caller's arrays,
+// at most kRayChunk rays at a time through buffers that the scene keeps (at most 62 MB).
+constexpr int kRayChunk = 1 << 20;
 
-void trace_batch(wr_scene &s, const float *rays, int n, int any_hit, std::vector<float> &out, unsigned long long *nv,
-                 unsigned long long *nt) {
+struct RayOutputs {   // host arrays, as RayAnswers
+    int *geom = nullptr, *prim = nullptr;
+    float *t = nullptr, *uv = nullptr, *normal = nullptr;
+    unsigned long long *visits = nullptr;
+};
+
+void trace_batch(wr_scene &s, const float *rays, int n, bool any_hit, const RayOutputs &out) {
     if (n < 0 || (n > 0 && !rays)) throw Error(WR_ERR_INVALID_ARGUMENT, "bad ray batch");
-    out.assign(size_t(n) * 12, 0.f);
+    if (out.visits) out.visits[0] = out.visits[1] = 0;
     if (n == 0) return;
-    DevBuf dr, dout, dvis;
-    dr.alloc(size_t(n) * 32);
-    dout.alloc(size_t(n) * 48);
-    dvis.alloc(8);
+    std::lock_guard<std::mutex> lock(s.ray_mutex);
     cudaStream_t st = s.stream;
-    WR_CUDA(cudaMemcpyAsync(dr.p, rays, size_t(n) * 32, cudaMemcpyHostToDevice, st));
-    WR_CUDA(cudaMemsetAsync(dvis.p, 0, 8, st));
-    int sms = 148;
-    WR_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, s.device));
-    const int grid = std::max(1, std::min(sms * 8, (n + wrd::kTraceBlock - 1) / wrd::kTraceBlock));
-    wrk::launch_trace_batch(scene_for_queries(s), dr.as<float4>(), uint32_t(n), any_hit, dout.as<float4>(),
-                            (nv || nt) ? dvis.as<uint32_t>() : nullptr, grid, st);
-    WR_CUDA(cudaGetLastError());
-    WR_CUDA(cudaMemcpyAsync(out.data(), dout.p, size_t(n) * 48, cudaMemcpyDeviceToHost, st));
-    uint32_t vis[2] = {0, 0};
-    WR_CUDA(cudaMemcpyAsync(vis, dvis.p, 8, cudaMemcpyDeviceToHost, st));
+    const int chunk = std::min(n, kRayChunk);
+    s.q_rays.alloc(size_t(chunk) * 32);
+    // the answers lie one array after another
+    const size_t words = (out.geom ? 1 : 0) + (out.prim ? 1 : 0) + (out.t ? 1 : 0) + (out.uv ? 2 : 0) + (out.normal ? 3 : 0);
+    s.q_answers.alloc(std::max<size_t>(size_t(chunk) * words * 4, 16));
+    unsigned long long *visits = nullptr;
+    if (out.visits) {
+        visits = s.q_answers.as<unsigned long long>();
+        WR_CUDA(cudaMemsetAsync(visits, 0, 16, st));
+    }
+    const int sms = sm_count(s);
+    for (int first = 0; first < n; first += chunk) {
+        const int m = std::min(chunk, n - first);
+        WR_CUDA(cudaMemcpyAsync(s.q_rays.p, rays + 8 * size_t(first), size_t(m) * 32, cudaMemcpyHostToDevice, st));
+        wrd::RayAnswers a{};
+        a.visits = visits;
+        struct Back { void *to; const void *from; size_t bytes; };
+        std::vector<Back> back;
+        float *next = s.q_answers.as<float>();
+        auto take = [&](void *host, int per_ray) -> float * {
+            if (!host) return nullptr;
+            float *dev = next;
+            next += size_t(chunk) * per_ray;
+            back.push_back({static_cast<float *>(host) + size_t(first) * per_ray, dev, size_t(m) * per_ray * 4});
+            return dev;
+        };
+        a.uv = reinterpret_cast<float2 *>(take(out.uv, 2));   // first: 8-byte aligned
+        a.geom = reinterpret_cast<int *>(take(out.geom, 1));
+        a.prim = reinterpret_cast<int *>(take(out.prim, 1));
+        a.t = take(out.t, 1);
+        a.normal = take(out.normal, 3);
+        wrk::launch_trace_batch(s.dev, s.q_rays.as<float4>(), uint32_t(m), any_hit, a, sms, st);
+        WR_CUDA(cudaGetLastError());
+        for (const Back &b : back) WR_CUDA(cudaMemcpyAsync(b.to, b.from, b.bytes, cudaMemcpyDeviceToHost, st));
+        // the buffers are free for the next chunk once the copies, which follow the kernel, are done
+    }
+    if (visits) WR_CUDA(cudaMemcpyAsync(out.visits, visits, 16, cudaMemcpyDeviceToHost, st));
     WR_CUDA(cudaStreamSynchronize(st));
-    if (nv) *nv = vis[0];
-    if (nt) *nt = vis[1];
 }
 
 // build options checked, bvh_width 0 replaced by the default
@@ -1625,18 +1656,12 @@ int wr_guide_train(wr_scene *s, const float *records, int n, int steps, int batc
 int wr_trace_closest(wr_scene *s, const float *rays, int n, int *geom_id, int *prim_id, float *t, float *uv) {
     if (!s || (n > 0 && (!geom_id || !prim_id || !t))) { g_last_error = "null argument"; return WR_ERR_INVALID_ARGUMENT; }
     try {
-        std::vector<float> out;
-        trace_batch(*s, rays, n, 0, out, nullptr, nullptr);
-        for (int i = 0; i < n; ++i) {
-            const float *o = &out[12 * size_t(i)];
-            uint32_t g, p;
-            memcpy(&g, &o[0], 4);
-            memcpy(&p, &o[1], 4);
-            geom_id[i] = g == wrd::MISS ? -1 : int(g);
-            prim_id[i] = p == wrd::MISS ? -1 : int(p);
-            t[i] = o[2];
-            if (uv) { uv[2 * i] = o[4]; uv[2 * i + 1] = o[5]; }
-        }
+        RayOutputs out;
+        out.geom = geom_id;
+        out.prim = prim_id;
+        out.t = t;
+        out.uv = uv;
+        trace_batch(*s, rays, n, false, out);
         return WR_OK;
     } catch (const Error &e) {
         return fail(e);
@@ -1649,18 +1674,12 @@ int wr_trace_hits(wr_scene *s, const float *rays, int n, int *geom_id, int *prim
         return WR_ERR_INVALID_ARGUMENT;
     }
     try {
-        std::vector<float> out;
-        trace_batch(*s, rays, n, 0, out, nullptr, nullptr);
-        for (int i = 0; i < n; ++i) {
-            const float *o = &out[12 * size_t(i)];
-            uint32_t g, p;
-            memcpy(&g, &o[0], 4);
-            memcpy(&p, &o[1], 4);
-            geom_id[i] = g == wrd::MISS ? -1 : int(g);
-            prim_id[i] = p == wrd::MISS ? -1 : int(p);
-            t[i] = o[2];
-            for (int k = 0; k < 3; ++k) normal[3 * i + k] = o[8 + k];
-        }
+        RayOutputs out;
+        out.geom = geom_id;
+        out.prim = prim_id;
+        out.t = t;
+        out.normal = normal;
+        trace_batch(*s, rays, n, false, out);
         return WR_OK;
     } catch (const Error &e) {
         return fail(e);
@@ -1670,13 +1689,9 @@ int wr_trace_hits(wr_scene *s, const float *rays, int n, int *geom_id, int *prim
 int wr_trace_occluded(wr_scene *s, const float *rays, int n, int *occluded) {
     if (!s || (n > 0 && !occluded)) { g_last_error = "null argument"; return WR_ERR_INVALID_ARGUMENT; }
     try {
-        std::vector<float> out;
-        trace_batch(*s, rays, n, 1, out, nullptr, nullptr);
-        for (int i = 0; i < n; ++i) {
-            uint32_t g;
-            memcpy(&g, &out[12 * size_t(i)], 4);
-            occluded[i] = g == wrd::MISS ? 0 : 1;
-        }
+        RayOutputs out;
+        out.geom = occluded;
+        trace_batch(*s, rays, n, true, out);
         return WR_OK;
     } catch (const Error &e) {
         return fail(e);
@@ -1687,8 +1702,12 @@ int wr_trace_stats(wr_scene *s, const float *rays, int n, int any_hit, unsigned 
                    unsigned long long *tri_tests) {
     if (!s || !node_visits || !tri_tests) { g_last_error = "null argument"; return WR_ERR_INVALID_ARGUMENT; }
     try {
-        std::vector<float> out;
-        trace_batch(*s, rays, n, any_hit, out, node_visits, tri_tests);
+        unsigned long long visits[2] = {0, 0};
+        RayOutputs out;
+        out.visits = visits;
+        trace_batch(*s, rays, n, any_hit != 0, out);
+        *node_visits = visits[0];
+        *tri_tests = visits[1];
         return WR_OK;
     } catch (const Error &e) {
         return fail(e);

@@ -119,6 +119,15 @@ struct DevScene {
     const float *env_col_pdf;
 };
 
+// answers of a ray batch in device memory, one array per quantity (null: not wanted)
+struct RayAnswers {
+    int *geom, *prim;             // closest: mesh and primitive number, -1 on a miss; occlusion: 0 / 1 in geom
+    float *t;                     // closest: distance, +inf on a miss
+    float2 *uv;                   // closest: a triangle's barycentrics
+    float *normal;                // closest: unit geometry normal, 3 per ray
+    unsigned long long *visits;   // statistics: total node visits and triangle tests, and no answers
+};
+
 // ------------------------------------------------------------- float3 ----
 struct f3 { float x, y, z; };
 __device__ __forceinline__ f3 mk(float x, float y, float z) { return {x, y, z}; }

@@ -19,6 +19,7 @@
 // Arithmetic is FP32; FP64 is used for the film and for building the light /
 // environment CDF tables (the prefix sums at the end of this file).
 
+#include <algorithm>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -1028,51 +1029,56 @@ __global__ void k_resolve(const double *film, double *out, uint32_t total_pix, c
 }
 
 // ----------------------------------------------------------- ray batches ----
-// rays: n x 8 floats (ox, oy, oz, tnear, dx, dy, dz, tfar)
-// out: 3 float4 per ray -- (geomID, primID, t, leaf index), (u, v, 0, 0) with the triangle's
-// barycentrics (zero on a patch, whose texture coordinate the reference leaves at zero), and
-// (unit geometry normal, 0)
-template <bool PHONG, bool WIDE>
-__global__ void __launch_bounds__(kTraceBlock) k_trace_batch(DevScene s, const float4 *rays, uint32_t n, int any_hit,
-                                                           float4 *out, uint32_t *visits) {
+// rays: n x 8 floats (ox, oy, oz, tnear, dx, dy, dz, tfar). The answers are written as the queries
+// return them (RayAnswers, one array per quantity), so the host copies them straight into the caller's
+// arrays: 20 bytes per ray for closest, 24 with normals, 4 for occlusion, where a 48-byte record of
+// all of them had to be copied and taken apart on the host (29 ms for a million rays). COUNT: node
+// visits and triangle tests (the statistics query) instead of answers.
+template <bool ANY_HIT, bool PHONG, bool WIDE, bool COUNT>
+__global__ void __launch_bounds__(kTraceBlock) k_trace_batch(DevScene s, const float4 *rays, uint32_t n, RayAnswers out) {
     extern __shared__ uint32_t stack[];
     TraceStack st;
     st.init(stack + threadIdx.x, kTraceBlock);
     uint32_t nv = 0, nt = 0;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const float4 a = rays[2 * i], b = rays[2 * i + 1];
+        const float4 a = __ldcs(rays + 2 * size_t(i)), b = __ldcs(rays + 2 * size_t(i) + 1);
         float t, bu = 0.f, bv = 0.f;
         uint32_t tri;
         bool hit;
-        if (WIDE && any_hit)
-            hit = traverse_w8<true, PHONG>(s.wnodes, s.tris, xyz(a), xyz(b), a.w, b.w, st, t, tri, bu, bv, nv, nt,
-                                           s.patches);
-        else if (WIDE)
-            hit = traverse_w8<false, PHONG>(s.wnodes, s.tris, xyz(a), xyz(b), a.w, b.w, st, t, tri, bu, bv, nv, nt,
-                                            s.patches);
-        else if (any_hit)
-            hit = traverse<true, PHONG>(s.nodes, s.tris, xyz(a), xyz(b), a.w, b.w, st, t, tri, bu, bv, nv, nt,
-                                        s.patches);
+        if (WIDE)
+            hit = traverse_w8<ANY_HIT, PHONG, COUNT>(s.wnodes, s.tris, xyz(a), xyz(b), a.w, b.w, st, t, tri, bu, bv, nv, nt,
+                                                     s.patches);
         else
-            hit = traverse<false, PHONG>(s.nodes, s.tris, xyz(a), xyz(b), a.w, b.w, st, t, tri, bu, bv, nv, nt,
-                                         s.patches);
-        uint32_t gid = MISS, pid = MISS;
+            hit = traverse<ANY_HIT, PHONG, COUNT>(s.nodes, s.tris, xyz(a), xyz(b), a.w, b.w, st, t, tri, bu, bv, nv, nt,
+                                                  s.patches);
+        if (COUNT) continue;
+        if (ANY_HIT) {
+            out.geom[i] = hit ? 1 : 0;
+            continue;
+        }
+        int gid = -1, pid = -1;
         f3 ng = mk(0.f, 0.f, 0.f);
         if (hit) {
             const float4 ta = __ldg(s.tris + 3 * tri), tb = __ldg(s.tris + 3 * tri + 1), tc = __ldg(s.tris + 3 * tri + 2);
-            gid = __float_as_uint(tb.w);
-            pid = __float_as_uint(tc.w);
-            ng = surface_normal(ta, tb, tc, bu, bv);
+            gid = __float_as_int(tb.w);
+            pid = __float_as_int(tc.w);
+            if (out.normal) ng = surface_normal(ta, tb, tc, bu, bv);
+            // a patch hit's slots held its normal; the reference leaves its texture coordinate at zero
             if (__float_as_uint(ta.w) & wrp::kPatchFlag) { bu = 0.f; bv = 0.f; }
         }
-        out[3 * i] = make_float4(__uint_as_float(gid), __uint_as_float(pid), hit ? t : __int_as_float(0x7f800000),
-                                 __uint_as_float(tri));
-        out[3 * i + 1] = make_float4(bu, bv, 0.f, 0.f);
-        out[3 * i + 2] = make_float4(ng.x, ng.y, ng.z, 0.f);
+        out.geom[i] = gid;
+        out.prim[i] = pid;
+        out.t[i] = hit ? t : __int_as_float(0x7f800000);
+        if (out.uv) out.uv[i] = make_float2(hit ? bu : 0.f, hit ? bv : 0.f);
+        if (out.normal) {
+            out.normal[3 * size_t(i)] = ng.x;
+            out.normal[3 * size_t(i) + 1] = ng.y;
+            out.normal[3 * size_t(i) + 2] = ng.z;
+        }
     }
-    if (visits) {
-        atomicAdd(visits, nv);
-        atomicAdd(visits + 1, nt);
+    if (COUNT) {
+        atomicAdd(out.visits, (unsigned long long)nv);
+        atomicAdd(out.visits + 1, (unsigned long long)nt);
     }
 }
 
@@ -1315,13 +1321,33 @@ void launch_resolve(const double *film, double *out, const RenderLaunch &r, cuda
     launch_chained(k_resolve, 592, 256, 0, st, r.chain != 0, film, out, r.total_pix, r.jobs, r.num_jobs, r.job0);
 }
 
-void launch_trace_batch(const DevScene &s, const float4 *rays, uint32_t n, int any_hit, float4 *out, uint32_t *visits,
-                        int grid, cudaStream_t st) {
-    const size_t bytes = size_t(s.stack_words) * kTraceBlock * 4;   // at most 33 KB
-    if (s.patches && s.wnodes) k_trace_batch<true, true><<<grid, kTraceBlock, bytes, st>>>(s, rays, n, any_hit, out, visits);
-    else if (s.patches) k_trace_batch<true, false><<<grid, kTraceBlock, bytes, st>>>(s, rays, n, any_hit, out, visits);
-    else if (s.wnodes) k_trace_batch<false, true><<<grid, kTraceBlock, bytes, st>>>(s, rays, n, any_hit, out, visits);
-    else k_trace_batch<false, false><<<grid, kTraceBlock, bytes, st>>>(s, rays, n, any_hit, out, visits);
+template <bool ANY_HIT, bool PHONG, bool WIDE, bool COUNT>
+void launch_trace_batch_4(const DevScene &s, const float4 *rays, uint32_t n, const RayAnswers &out, int sms,
+                          cudaStream_t st) {
+    auto *kernel = k_trace_batch<ANY_HIT, PHONG, WIDE, COUNT>;
+    const size_t bytes = stack_bytes(kernel, s, kTraceBlock);
+    int nb = 0;
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kernel, kTraceBlock, bytes);
+    const uint32_t grid = std::min(uint32_t(sms) * uint32_t(std::max(nb, 1)), (n + kTraceBlock - 1) / kTraceBlock);
+    kernel<<<grid, kTraceBlock, bytes, st>>>(s, rays, n, out);
+}
+
+template <bool ANY_HIT, bool COUNT>
+void launch_trace_batch_2(const DevScene &s, const float4 *rays, uint32_t n, const RayAnswers &out, int sms,
+                          cudaStream_t st) {
+    if (s.patches && s.wnodes) launch_trace_batch_4<ANY_HIT, true, true, COUNT>(s, rays, n, out, sms, st);
+    else if (s.patches) launch_trace_batch_4<ANY_HIT, true, false, COUNT>(s, rays, n, out, sms, st);
+    else if (s.wnodes) launch_trace_batch_4<ANY_HIT, false, true, COUNT>(s, rays, n, out, sms, st);
+    else launch_trace_batch_4<ANY_HIT, false, false, COUNT>(s, rays, n, out, sms, st);
+}
+
+void launch_trace_batch(const DevScene &s, const float4 *rays, uint32_t n, bool any_hit, const RayAnswers &out, int sms,
+                        cudaStream_t st) {
+    if (n == 0) return;
+    if (any_hit && out.visits) launch_trace_batch_2<true, true>(s, rays, n, out, sms, st);
+    else if (any_hit) launch_trace_batch_2<true, false>(s, rays, n, out, sms, st);
+    else if (out.visits) launch_trace_batch_2<false, true>(s, rays, n, out, sms, st);
+    else launch_trace_batch_2<false, false>(s, rays, n, out, sms, st);
 }
 
 void launch_cdf_build(const double *weights, const uint32_t *offsets, uint32_t ntables, float *cdf, float *pdf,

@@ -64,8 +64,8 @@ void launch_iteration_fused(const DevScene &s, const WaveBuffers &b, const Rende
                             cudaStream_t st);
 void launch_shadow_flush(const DevScene &s, const WaveBuffers &b, const RenderLaunch &r, cudaStream_t st);
 void launch_resolve(const double *film, double *out, const RenderLaunch &r, cudaStream_t st);
-void launch_trace_batch(const DevScene &s, const float4 *rays, uint32_t n, int any_hit, float4 *out, uint32_t *visits,
-                        int grid, cudaStream_t st);
+void launch_trace_batch(const DevScene &s, const float4 *rays, uint32_t n, bool any_hit, const RayAnswers &out, int sms,
+                        cudaStream_t st);
 void launch_cdf_build(const double *weights, const uint32_t *offsets, uint32_t ntables, float *cdf, float *pdf,
                       double *sums, cudaStream_t st);
 void launch_env_weights(const float4 *texels, int w, int h, double *out, cudaStream_t st);

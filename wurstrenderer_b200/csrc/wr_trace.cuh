@@ -271,7 +271,7 @@ __device__ __forceinline__ bool traverse_steps(const float4 *__restrict__ nodes,
 }
 
 // one whole query (the k_trace_batch path)
-template <bool ANY_HIT, bool PHONG>
+template <bool ANY_HIT, bool PHONG, bool COUNT>
 __device__ __forceinline__ bool traverse(const float4 *__restrict__ nodes, const float4 *__restrict__ tris, f3 o,
                                          f3 d, float tmin, float tmax, TraceStack &st, float &t, uint32_t &tri,
                                          float &bu, float &bv, uint32_t &nv, uint32_t &nt, const double *patches) {
@@ -281,7 +281,7 @@ __device__ __forceinline__ bool traverse(const float4 *__restrict__ nodes, const
     tri = MISS;
     t = tmax;
     st.clear();
-    traverse_steps<ANY_HIT, PHONG, true, true>(nodes, tris, r, tmin, t, tri, bu, bv, node, leaf, st, nv, nt, 0, patches,
+    traverse_steps<ANY_HIT, PHONG, !ANY_HIT, COUNT>(nodes, tris, r, tmin, t, tri, bu, bv, node, leaf, st, nv, nt, 0, patches,
                                                pr);
     return tri != MISS;
 }
@@ -428,7 +428,7 @@ __device__ __forceinline__ uint32_t ray_octant(f3 d) {
 }
 
 // one whole query on the compressed 8-wide BVH (the k_trace_batch path)
-template <bool ANY_HIT, bool PHONG>
+template <bool ANY_HIT, bool PHONG, bool COUNT>
 __device__ __forceinline__ bool traverse_w8(const uint4 *__restrict__ wnodes, const float4 *__restrict__ tris, f3 o,
                                             f3 d, float tmin, float tmax, TraceStack &st, float &t, uint32_t &tri,
                                             float &bu, float &bv, uint32_t &nv, uint32_t &nt, const double *patches) {
@@ -438,7 +438,7 @@ __device__ __forceinline__ bool traverse_w8(const uint4 *__restrict__ wnodes, co
     tri = MISS;
     t = tmax;
     st.clear();
-    traverse_steps_w8<ANY_HIT, PHONG, true, true>(wnodes, tris, r, ray_octant(d), tmin, t, tri, bu, bv, ws, st, nv, nt,
+    traverse_steps_w8<ANY_HIT, PHONG, !ANY_HIT, COUNT>(wnodes, tris, r, ray_octant(d), tmin, t, tri, bu, bv, ws, st, nv, nt,
                                                   0, patches, pr);
     return tri != MISS;
 }
