@@ -924,32 +924,34 @@ uint32_t shuffle_stride(uint32_t n) {
 double train_records(wr_scene &s, const float4 *records, uint32_t n, uint32_t batch, int max_steps, float lr,
                      float c_max, std::vector<double> *per_step, unsigned long long *steps_out) {
     cudaStream_t st = s.stream;
-    s.g_loss.alloc(8 * 2);
     const uint32_t stride = shuffle_stride(n);
-    const int steps = max_steps > 0 ? max_steps : int((n + batch - 1) / batch);
-    double total = 0.0;
-    WR_CUDA(cudaMemsetAsync(s.g_loss.p, 0, 8, st));
-    for (int k = 0; k < steps && n > 0; ++k) {
+    const int steps = n == 0 ? 0 : max_steps > 0 ? max_steps : int((n + batch - 1) / batch);
+    // one sum for all steps, or one per step, read back together after the last: no step waits for
+    // the host (32 steps with a read-back each took 1.32 ms)
+    const size_t sums = per_step ? size_t(std::max(steps, 1)) : 1;
+    s.g_loss.alloc(std::max<size_t>(sums, 2) * 8);
+    double *loss = s.g_loss.as<double>();
+    WR_CUDA(cudaMemsetAsync(loss, 0, sums * 8, st));
+    std::vector<uint32_t> counts;
+    for (int k = 0; k < steps; ++k) {
         const uint32_t first = uint32_t((uint64_t(k) * batch) % n);
         const uint32_t cnt = std::min(batch, n - first);
-        if (per_step) WR_CUDA(cudaMemsetAsync(s.g_loss.p, 0, 8, st));
         // each kernel may be scheduled while the one before it ends (its set-up and the first
         // records' gather overlap that kernel); it waits for it before reading its results
         const int nslots = wrg::guide_gradient(s.guide, records, first + cnt, first, n, stride, c_max,
-                                               s.g_loss.as<double>(), st, k > 0 && !per_step);
+                                               per_step ? loss + k : loss, st, k > 0);
         wrg::guide_adam(s.guide, lr, 1.f / float(cnt), ++s.guide_step, nslots, st, true);
-        if (per_step) {
-            double l = 0.0;
-            WR_CUDA(cudaMemcpyAsync(&l, s.g_loss.p, 8, cudaMemcpyDeviceToHost, st));
-            WR_CUDA(cudaStreamSynchronize(st));
-            per_step->push_back(l / double(cnt));
-            total += l;
-        }
+        if (per_step) counts.push_back(cnt);
         if (steps_out) ++*steps_out;
     }
-    if (!per_step) {
-        WR_CUDA(cudaMemcpyAsync(&total, s.g_loss.p, 8, cudaMemcpyDeviceToHost, st));
-        WR_CUDA(cudaStreamSynchronize(st));
+    std::vector<double> sum(sums);
+    WR_CUDA(cudaMemcpyAsync(sum.data(), loss, sums * 8, cudaMemcpyDeviceToHost, st));
+    WR_CUDA(cudaStreamSynchronize(st));
+    double total = 0.0;
+    if (!per_step) total = sum[0];
+    for (size_t k = 0; k < counts.size(); ++k) {
+        per_step->push_back(sum[k] / double(counts[k]));
+        total += sum[k];
     }
     check_guide_status(s);
     return total;
@@ -1585,22 +1587,10 @@ int wr_guide_eval(wr_scene *s, const float *rows, int n, float *lobes) {
         WR_CUDA(cudaMemcpyAsync(s->g_scratch.p, rows, size_t(n) * 9 * 4, cudaMemcpyHostToDevice, st));
         wrg::guide_infer_rows(s->guide, s->g_scratch.as<float>(), uint32_t(n), s->g_scratch2.as<float4>(), sm_count(*s),
                               st);
-        std::vector<float4> out(size_t(n) * wrg::kLobeFloat4);
-        WR_CUDA(cudaMemcpyAsync(out.data(), s->g_scratch2.p, out.size() * 16, cudaMemcpyDeviceToHost, st));
-        WR_CUDA(cudaStreamSynchronize(st));
-        check_guide_status(*s);
-        for (int i = 0; i < n; ++i) {
-            const float4 *L = &out[size_t(i) * wrg::kLobeFloat4];
-            float *o = lobes + 40 * size_t(i);
-            for (int k = 0; k < 8; ++k) {
-                o[4 * k + 0] = L[k].x;
-                o[4 * k + 1] = L[k].y;
-                o[4 * k + 2] = L[k].z;
-                o[4 * k + 3] = L[k].w;
-            }
-            const float w[8] = {L[8].x, L[8].y, L[8].z, L[8].w, L[9].x, L[9].y, L[9].z, L[9].w};
-            for (int k = 0; k < 8; ++k) o[32 + k] = w[k];
-        }
+        // the kernel's rows (8 x axis and sharpness, then 8 weights) are the caller's 40 floats
+        static_assert(wrg::kLobeFloat4 * 4 == 40, "a lobe row is 40 floats");
+        WR_CUDA(cudaMemcpyAsync(lobes, s->g_scratch2.p, size_t(n) * wrg::kLobeFloat4 * 16, cudaMemcpyDeviceToHost, st));
+        check_guide_status(*s);   // waits for the copy
         return WR_OK;
     } catch (const Error &e) {
         return fail(e);
