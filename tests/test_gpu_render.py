@@ -320,3 +320,37 @@ def test_one_wave_renders_match_graphs(wr_lib, nverts, integrator):
         profiled = sc.render(profile=3, **kw)
     assert np.allclose(chained, graph, rtol=1e-9, atol=1e-12)
     assert np.allclose(chained, profiled, rtol=1e-9, atol=1e-12)
+
+
+@pytest.mark.parametrize("res", [[295, 295], [296, 296], [512, 401]])   # below, above and well above a direct copy
+def test_images_reach_the_host_whole(wr_lib, res):
+    """The film's way to the host: by the driver or in shared pieces, into fresh and pinned memory, and
+    from several threads at once (each with a scene of its own)."""
+    import json
+    import threading
+    import torch
+    path, _ = golden_scene("cornell")
+    cam = json.loads(open(path).read())["camera"]
+    cam["resolution"] = res
+    n = 3
+    want, got = [None] * n, [None] * n
+    scenes_ = [wr_lib.Scene.from_file(path) for _ in range(n)]
+    for k, sc in enumerate(scenes_):
+        sc.set_camera(json.dumps(cam))
+        want[k] = sc.render(spp=1, seed=k, out=torch.empty(res[1], res[0], 3, dtype=torch.float64,
+                                                           pin_memory=True).numpy()).copy()
+
+    def job(k):
+        got[k] = [scenes_[k].render(spp=1, seed=k) for _ in range(3)]
+
+    threads = [threading.Thread(target=job, args=(k,)) for k in range(n)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for k in range(n):
+        assert want[k].shape == (res[1], res[0], 3) and want[k].any()
+        for im in got[k]:
+            assert np.allclose(im, want[k], rtol=1e-9, atol=1e-12)
+    for sc in scenes_:
+        sc.close()

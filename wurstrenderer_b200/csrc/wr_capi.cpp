@@ -27,6 +27,7 @@
 #include "wr_host.h"
 #include "wr_kernels.h"
 #include "wr_phong.cuh"
+#include "wr_staging.h"
 
 using wr::Error;
 
@@ -101,6 +102,7 @@ struct wr_scene {
     uint32_t w_guide_capacity = 0, w_record_capacity = 0;
     uint32_t w_capacity = 0;
     size_t w_npix = 0;
+    std::shared_ptr<wr::Staging> staging = wr::Staging::shared();
     uint32_t *pinned = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     wr_render_stats stats{};
@@ -820,8 +822,8 @@ void render_jobs(wr_scene &s, const std::vector<HostJob> &jobs, const wr_render_
     }
     if (!desc.use_graph || one_wave || profile) WR_CUDA(cudaEventRecord(s.ev1, st));
     WR_CUDA(cudaMemcpyAsync(s.pinned, b.ctr, wrd::CTR_COUNT * 4, cudaMemcpyDeviceToHost, st));
-    if (out_on_host && out) WR_CUDA(cudaMemcpyAsync(out, dst, total_pix * 3 * 8, cudaMemcpyDeviceToHost, st));
     if (po.record) WR_CUDA(cudaMemcpyAsync(s.pinned + 12, b.rec_count, 4, cudaMemcpyDeviceToHost, st));
+    if (out_on_host && out) WR_CUDA(s.staging->to_host(out, dst, total_pix * 3 * 8, st));
     WR_CUDA(cudaStreamSynchronize(st));
     if (trace && (s.pinned[wrd::CTR_TIMEOUT] || !s.pinned[wrd::CTR_DONE])) throw Error(WR_ERR_TIMEOUT, "wavefront did not drain within the iteration bound");
     if (trace && s.pinned[wrd::CTR_OVERFLOW]) throw Error(WR_ERR_CUDA, "shadow queue overflow");
@@ -1162,7 +1164,7 @@ void trace_batch(wr_scene &s, const float *rays, int n, bool any_hit, const RayO
     const int sms = sm_count(s);
     for (int first = 0; first < n; first += chunk) {
         const int m = std::min(chunk, n - first);
-        WR_CUDA(cudaMemcpyAsync(s.q_rays.p, rays + 8 * size_t(first), size_t(m) * 32, cudaMemcpyHostToDevice, st));
+        WR_CUDA(s.staging->to_device(s.q_rays.p, rays + 8 * size_t(first), size_t(m) * 32, st));
         wrd::RayAnswers a{};
         a.visits = visits;
         struct Back { void *to; const void *from; size_t bytes; };
@@ -1182,7 +1184,7 @@ void trace_batch(wr_scene &s, const float *rays, int n, bool any_hit, const RayO
         a.normal = take(out.normal, 3);
         wrk::launch_trace_batch(s.dev, s.q_rays.as<float4>(), uint32_t(m), any_hit, a, sms, st);
         WR_CUDA(cudaGetLastError());
-        for (const Back &b : back) WR_CUDA(cudaMemcpyAsync(b.to, b.from, b.bytes, cudaMemcpyDeviceToHost, st));
+        for (const Back &b : back) WR_CUDA(s.staging->to_host(b.to, b.from, b.bytes, st));
         // the buffers are free for the next chunk once the copies, which follow the kernel, are done
     }
     if (visits) WR_CUDA(cudaMemcpyAsync(out.visits, visits, 16, cudaMemcpyDeviceToHost, st));
@@ -1587,13 +1589,13 @@ int wr_guide_eval(wr_scene *s, const float *rows, int n, float *lobes) {
         cudaStream_t st = s->stream;
         s->g_scratch.alloc(size_t(n) * 9 * 4);
         s->g_scratch2.alloc(size_t(n) * wrg::kLobeFloat4 * 16);
-        WR_CUDA(cudaMemcpyAsync(s->g_scratch.p, rows, size_t(n) * 9 * 4, cudaMemcpyHostToDevice, st));
+        WR_CUDA(s->staging->to_device(s->g_scratch.p, rows, size_t(n) * 9 * 4, st));
         wrg::guide_infer_rows(s->guide, s->g_scratch.as<float>(), uint32_t(n), s->g_scratch2.as<float4>(), sm_count(*s),
                               st);
         // the kernel's rows (8 x axis and sharpness, then 8 weights) are the caller's 40 floats
         static_assert(wrg::kLobeFloat4 * 4 == 40, "a lobe row is 40 floats");
-        WR_CUDA(cudaMemcpyAsync(lobes, s->g_scratch2.p, size_t(n) * wrg::kLobeFloat4 * 16, cudaMemcpyDeviceToHost, st));
-        check_guide_status(*s);   // waits for the copy
+        WR_CUDA(s->staging->to_host(lobes, s->g_scratch2.p, size_t(n) * wrg::kLobeFloat4 * 16, st));
+        check_guide_status(*s);
         return WR_OK;
     } catch (const Error &e) {
         return fail(e);
