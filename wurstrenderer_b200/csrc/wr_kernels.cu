@@ -386,18 +386,18 @@ __device__ __forceinline__ void film_add(const WaveArgs &w, uint32_t slot, f3 c)
 // loop and its idle lanes take the next rays of the queue (one atomic per warp), so that
 // SIMD lanes are not left idle while a few long rays finish (Aila & Laine, HPG 2009). Once
 // the queue is exhausted the remaining rays run to completion.
-//   SHADOW = false: extend -- closest hit of every live path into the hit records
-//   SHADOW = true:  shadow -- any hit of every queued shadow ray; unoccluded contributions
+//   shadow = false: extend -- closest hit of every live path into the hit records
+//   shadow = true:  shadow -- any hit of every queued shadow ray; unoccluded contributions
 //                   are added to the FP64 film (and to the path's training records)
 
 //   count_ctr: the counter holding the queue length (CTR_ACTIVE; CTR_SHADOW, or
 //              CTR_SHADOW_PENDING for the previous iteration's queue)
 
 //   COUNT: node visits and triangle tests are counted into w.prof (profiled renders)
-template <int BLOCK, bool SHADOW, bool PHONG, bool WIDE, bool COUNT>
-__device__ __forceinline__ void trace_queue(const DevScene &s, const WaveArgs &w, uint32_t *stack, int count_ctr) {
-    const uint32_t n = SHADOW ? min(w.ctr[count_ctr], w.shadow_capacity) : w.ctr[count_ctr];
-    uint32_t *fetch = w.ctr + (SHADOW ? CTR_SHADOW_FETCH : CTR_EXTEND_FETCH);
+template <int BLOCK, bool PHONG, bool WIDE, bool COUNT>
+__device__ __forceinline__ void trace_queue(const DevScene &s, const WaveArgs &w, uint32_t *stack, int count_ctr, const bool shadow) {
+    const uint32_t n = shadow ? min(w.ctr[count_ctr], w.shadow_capacity) : w.ctr[count_ctr];
+    uint32_t *fetch = w.ctr + (shadow ? CTR_SHADOW_FETCH : CTR_EXTEND_FETCH);
     TraceStack st;
     st.init(stack + threadIdx.x, BLOCK);
     RayPre r{};
@@ -405,6 +405,7 @@ __device__ __forceinline__ void trace_queue(const DevScene &s, const WaveArgs &w
     float t = 0.f, bu = 0.f, bv = 0.f;
     uint32_t tri = MISS, ray = 0, nv = 0, nt = 0;
     int node = kTraceDone, leaf = 0;
+    PatchState ps{0u, 0u, MISS};
     WideState ws{-1, 0u, 0u, 0u};   // WIDE: compressed 8-wide traversal state
     uint32_t oct = 0;
     bool busy = false, exhausted = false;
@@ -421,7 +422,7 @@ __device__ __forceinline__ void trace_queue(const DevScene &s, const WaveArgs &w
                 if (ray < n) {
                     float4 o, d;
                     float tmax;
-                    if (SHADOW) { o = __ldcs(&w.sq.o[ray]); d = __ldcs(&w.sq.d[ray]); tmax = o.w; }
+                    if (shadow) { o = __ldcs(&w.sq.o[ray]); d = __ldcs(&w.sq.d[ray]); tmax = o.w; }
                     else { o = w.cur.o[ray]; d = w.cur.d[ray]; tmax = __int_as_float(0x7f800000); }
                     r = ray_setup(xyz(o), xyz(d));
                     if (PHONG) pr = PatchRay{o.x, o.y, o.z, d.x, d.y, d.z};
@@ -442,15 +443,23 @@ __device__ __forceinline__ void trace_queue(const DevScene &s, const WaveArgs &w
         bool finished = false;
         if (busy) {
             if (WIDE)
-                finished = traverse_steps_w8<SHADOW, PHONG, false, COUNT>(s.wnodes, s.tris, r, oct, kRayEps, t, tri, bu, bv, ws, st,
-                                                             nv, nt, min_active, s.patches, pr);
+                finished = shadow ? traverse_steps_w8<true, PHONG, false, COUNT>(s.wnodes, s.tris, r, oct, kRayEps, t, tri, bu, bv,
+                                                                                 ws, st, nv, nt, min_active, s.patches, pr)
+                                  : traverse_steps_w8<false, PHONG, false, COUNT>(s.wnodes, s.tris, r, oct, kRayEps, t, tri, bu, bv,
+                                                                                  ws, st, nv, nt, min_active, s.patches, pr);
+            else if (PHONG)
+                finished = traverse_patches<COUNT>(s.nodes, s.tris, s.patches, r, pr, shadow, kRayEps, t, tri, bu, bv, node, leaf,
+                                                   ps, st, nv, nt, min_active);
+            else if (shadow)
+                finished = traverse_steps<true, false, COUNT>(s.nodes, s.tris, r, kRayEps, t, tri, bu, bv, node, leaf, st, nv, nt,
+                                                              min_active);
             else
-                finished = traverse_steps<SHADOW, PHONG, false, COUNT>(s.nodes, s.tris, r, kRayEps, t, tri, bu, bv, node, leaf,
-                                                                       st, nv, nt, min_active, s.patches, pr);
+                finished = traverse_steps<false, false, COUNT>(s.nodes, s.tris, r, kRayEps, t, tri, bu, bv, node, leaf, st, nv, nt,
+                                                               min_active);
         }
         if (finished) {
             busy = false;
-            if (SHADOW) {
+            if (shadow) {
                 if (tri == MISS) {   // unoccluded
                     const float4 c = __ldcs(&w.sq.c[ray]);
                     film_add(w, __float_as_uint(__ldcs(&w.sq.d[ray]).w), mk(c.x, c.y, c.z));
@@ -464,10 +473,10 @@ __device__ __forceinline__ void trace_queue(const DevScene &s, const WaveArgs &w
     if (COUNT) {   // the whole warp leaves the loop together: one atomic per warp and counter
         const uint32_t wnv = __reduce_add_sync(0xffffffffu, nv), wnt = __reduce_add_sync(0xffffffffu, nt);
         if (lane == 0) {
-            atomicAdd(w.prof + (SHADOW ? 8 : 6), (unsigned long long)wnv);
-            atomicAdd(w.prof + (SHADOW ? 9 : 7), (unsigned long long)wnt);
+            atomicAdd(w.prof + (shadow ? 8 : 6), (unsigned long long)wnv);
+            atomicAdd(w.prof + (shadow ? 9 : 7), (unsigned long long)wnt);
         }
-        if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(w.prof + (SHADOW ? 3 : 0), (unsigned long long)n);
+        if (blockIdx.x == 0 && threadIdx.x == 0) atomicAdd(w.prof + (shadow ? 3 : 0), (unsigned long long)n);
     }
 }
 
@@ -476,7 +485,7 @@ template <int BLOCK, bool PHONG, bool WIDE, bool COUNT>
 __global__ void __launch_bounds__(BLOCK) k_extend(DevScene s, WaveArgs w) {
     chain_begin();
     extern __shared__ uint32_t stack[];
-    trace_queue<BLOCK, false, PHONG, WIDE, COUNT>(s, w, stack, CTR_ACTIVE);
+    trace_queue<BLOCK, PHONG, WIDE, COUNT>(s, w, stack, CTR_ACTIVE, false);
 }
 
 // lens point of a sample's camera vertex (ThinlensCamera::sampleWe0ByPdf, thinlens.h:121-136; the
@@ -956,7 +965,7 @@ template <int BLOCK, bool PHONG, bool WIDE, bool COUNT>
 __global__ void __launch_bounds__(BLOCK) k_shadow(DevScene s, WaveArgs w, int count_ctr) {
     chain_begin();
     extern __shared__ uint32_t stack[];
-    trace_queue<BLOCK, true, PHONG, WIDE, COUNT>(s, w, stack, count_ctr);
+    trace_queue<BLOCK, PHONG, WIDE, COUNT>(s, w, stack, count_ctr, true);
 }
 
 // Extend of this iteration and the shadow rays of the previous one in one persistent launch:
@@ -969,8 +978,14 @@ template <int BLOCK, bool PHONG, bool WIDE, bool COUNT>
 __device__ __forceinline__ void trace_pair(const DevScene &s, const WaveArgs &w) {
     chain_begin();
     extern __shared__ uint32_t stack[];
-    trace_queue<BLOCK, false, PHONG, WIDE, COUNT>(s, w, stack, CTR_ACTIVE);
-    trace_queue<BLOCK, true, PHONG, WIDE, COUNT>(s, w, stack, CTR_SHADOW_PENDING);
+    if (PHONG && !WIDE) {   // one copy of the FP64 patch test for both kinds of rays
+#pragma unroll 1
+        for (int k = 0; k < 2; ++k)
+            trace_queue<BLOCK, PHONG, WIDE, COUNT>(s, w, stack, k ? int(CTR_SHADOW_PENDING) : int(CTR_ACTIVE), k != 0);
+        return;
+    }
+    trace_queue<BLOCK, PHONG, WIDE, COUNT>(s, w, stack, CTR_ACTIVE, false);
+    trace_queue<BLOCK, PHONG, WIDE, COUNT>(s, w, stack, CTR_SHADOW_PENDING, true);
 }
 
 template <int BLOCK, bool WIDE, bool COUNT>
@@ -978,10 +993,11 @@ __global__ void __launch_bounds__(BLOCK) k_trace_pair(DevScene s, WaveArgs w) {
     trace_pair<BLOCK, false, WIDE, COUNT>(s, w);
 }
 
-// With Phong patches both FP64 patch tests in one kernel would take 190 registers (2 blocks of
-// 128 per SM); the bound keeps the 384 resident threads per SM of the separate kernels.
+// The FP64 patch test wants 222 registers, which leaves 256 resident threads per SM. Held to 168
+// registers (384 threads) it spills and takes 18.7 ms for a frame of 56,000 patches that takes 16.9
+// with all its registers; with 128 threads per SM it takes 25.4.
 template <int BLOCK, bool WIDE, bool COUNT>
-__global__ void __launch_bounds__(BLOCK, (384 / BLOCK > 0 ? 384 / BLOCK : 1)) k_trace_pair_phong(DevScene s, WaveArgs w) {
+__global__ void __launch_bounds__(BLOCK, 256 / BLOCK) k_trace_pair_phong(DevScene s, WaveArgs w) {
     trace_pair<BLOCK, true, WIDE, COUNT>(s, w);
 }
 

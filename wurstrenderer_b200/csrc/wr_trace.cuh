@@ -120,14 +120,10 @@ struct PatchRay {
     float ox, oy, oz, dx, dy, dz;
 };
 
-// leaf primitive i is a patch: its own box, then the FP64 test against (tmin, t]; on a hit
-// lowers t and stores the encoded normal in (bu, bv)
-__device__ __forceinline__ bool patch_leaf_test(const RayPre &r, const PatchRay &pr, const double *patches, uint32_t i,
-                                                float4 a, float4 b, float4 c, float tmin, float &t, float &bu,
-                                                float &bv) {
-    float lo[3], hi[3];
-    wrp::load_patch_box(patches, i, lo, hi);
-    if (box_entry(r, lo[0], hi[0], lo[1], hi[1], lo[2], hi[2], tmin, t) == __int_as_float(0x7f800000)) return false;
+// the FP64 test of patch i, whose own box the ray has passed, against (tmin, t]; on a hit lowers t and
+// stores the encoded normal in (bu, bv)
+__device__ __forceinline__ bool patch_test(const PatchRay &pr, const double *patches, uint32_t i, float4 a, float4 b,
+                                           float4 c, float tmin, float &t, float &bu, float &bv) {
     const wrp::Patch<wrp::Rd> P = wrp::load_patch(patches, i, a, b, c);
     wrp::Rd tm = wrp::Rd(double(t));
     wrp::V<wrp::Rd> n;
@@ -137,6 +133,16 @@ __device__ __forceinline__ bool patch_leaf_test(const RayPre &r, const PatchRay 
     bu = e.x;
     bv = e.y;
     return true;
+}
+
+// leaf primitive i is a patch: its own box, then the FP64 test
+__device__ __forceinline__ bool patch_leaf_test(const RayPre &r, const PatchRay &pr, const double *patches, uint32_t i,
+                                                float4 a, float4 b, float4 c, float tmin, float &t, float &bu,
+                                                float &bv) {
+    float lo[3], hi[3];
+    wrp::load_patch_box(patches, i, lo, hi);
+    if (box_entry(r, lo[0], hi[0], lo[1], hi[1], lo[2], hi[2], tmin, t) == __int_as_float(0x7f800000)) return false;
+    return patch_test(pr, patches, i, a, b, c, tmin, t, bu, bv);
 }
 
 // unit geometry normal of a hit on leaf primitive (a, b, c): the triangle's face normal,
@@ -201,12 +207,11 @@ struct TraceStack {
 // 44.7 ms for the 1.16M-triangle frame.
 constexpr int kLeafWait = 4;
 
-template <bool ANY_HIT, bool PHONG, bool UV, bool COUNT>
+template <bool ANY_HIT, bool UV, bool COUNT>
 __device__ __forceinline__ bool traverse_steps(const float4 *__restrict__ nodes, const float4 *__restrict__ tris,
                                                const RayPre &r, float tmin, float &t, uint32_t &tri, float &bu,
                                                float &bv, int &node, int &leaf, TraceStack &st, uint32_t &nv,
-                                               uint32_t &nt, int min_active, const double *patches = nullptr,
-                                               const PatchRay &pr = PatchRay{}) {
+                                               uint32_t &nt, int min_active) {
     while (node != kTraceDone) {
         while (uint32_t(node) < uint32_t(kTraceDone)) {   // an inner node
             float4 n0, n1, n2, n3;
@@ -234,23 +239,12 @@ __device__ __forceinline__ bool traverse_steps(const float4 *__restrict__ nodes,
                 const float4 b = __ldg(tris + 3 * i + 1);
                 const float4 c = __ldg(tris + 3 * i + 2);
                 if (COUNT) ++nt;
-                if (PHONG && (__float_as_uint(a.w) & wrp::kPatchFlag)) {
-                    if (patch_leaf_test(r, pr, patches, i, a, b, c, tmin, t, bu, bv)) {
-                        tri = i;
-                        if (ANY_HIT) {
-                            node = kTraceDone;
-                            leaf = 0;
-                            return true;
-                        }
-                    }
-                    continue;
-                }
                 float th, uh, vh;
                 if (tri_test(r, a, b, c, tmin, t, th, uh, vh)) {
                     if (ANY_HIT || th < t || tri == MISS) {
                         t = th;
                         tri = i;
-                        if (UV || PHONG) { bu = uh; bv = vh; }
+                        if (UV) { bu = uh; bv = vh; }
                     }
                     if (ANY_HIT) {
                         node = kTraceDone;
@@ -270,6 +264,101 @@ __device__ __forceinline__ bool traverse_steps(const float4 *__restrict__ nodes,
     return true;
 }
 
+// The same for scenes with Phong patches (ANY_HIT as an argument, so that a kernel that traces both
+// kinds of rays holds the FP64 patch test once). A patch test is some two thousand instructions, and
+// where every lane ran it as soon as it met a patch, 4.75 of 32 lanes ran it together and the warps'
+// different places in it thrashed the instruction cache. Here a lane whose patch passes its own box
+// holds it (`pend`) and waits, descending further where it can, until kPatchWait lanes of the warp hold
+// one or none can do anything else: 27.0 -> 18.9 ms for a frame of 56,000 patches (kPatchWait 1 / 8 / 12 /
+// 16 / 20: 19.6 / 18.7 / 18.9 / 18.8 / 19.0), 16.9 with the registers that the fused kernel then gives it.
+// The postponed leaf's remaining primitives are [cur, end).
+constexpr int kPatchWait = 12;
+
+struct PatchState {
+    uint32_t cur, end;   // primitives of the leaf in hand still to be tested
+    uint32_t pend;       // patch waiting for its FP64 test, MISS when none
+};
+
+template <bool COUNT>
+__device__ __forceinline__ bool traverse_patches(const float4 *__restrict__ nodes, const float4 *__restrict__ tris,
+                                                 const double *__restrict__ patches, const RayPre &r, const PatchRay &pr,
+                                                 bool any_hit, float tmin, float &t, uint32_t &tri, float &bu, float &bv,
+                                                 int &node, int &leaf, PatchState &ps, TraceStack &st, uint32_t &nv,
+                                                 uint32_t &nt, int min_active) {
+    while (node != kTraceDone || leaf < 0 || ps.cur < ps.end || ps.pend != MISS) {
+        while (uint32_t(node) < uint32_t(kTraceDone)) {
+            float4 n0, n1, n2, n3;
+            ld_node(nodes + 4 * node, n0, n1, n2, n3);
+            if (COUNT) ++nv;
+            const float e0 = box_entry(r, n0.x, n0.y, n0.z, n0.w, n2.x, n2.y, tmin, t);
+            const float e1 = box_entry(r, n1.x, n1.y, n1.z, n1.w, n2.z, n2.w, tmin, t);
+            const int c0 = __float_as_int(n3.x), c1 = __float_as_int(n3.y);
+            const bool h0 = e0 != __int_as_float(0x7f800000), h1 = e1 != __int_as_float(0x7f800000);
+            const bool swap = e1 < e0;
+            st.push_if(h0 && h1, swap ? c0 : c1);
+            node = swap ? c1 : c0;
+            st.pop_if(!h0 && !h1, node);
+            const bool take = node < 0 && leaf == 0;
+            leaf = take ? node : leaf;
+            st.pop_if(take, node);
+            if (__popc(__ballot_sync(__activemask(), leaf == 0)) < kLeafWait) break;
+        }
+        bool found = false;   // a hit that ends the ray (any_hit)
+        while (!found && ps.pend == MISS && (ps.cur < ps.end || leaf < 0)) {
+            if (ps.cur == ps.end) {   // the next leaf
+                ps.cur = uint32_t(leaf) & 0x07ffffffu;
+                ps.end = ps.cur + ((uint32_t(leaf) >> 27) & 0xfu) + 1u;
+                leaf = 0;
+                if (node < 0) {
+                    leaf = node;
+                    st.pop_if(true, node);
+                }
+            }
+            const uint32_t i = ps.cur++;
+            const float4 a = __ldg(tris + 3 * i + 0);
+            if (COUNT) ++nt;
+            if (__float_as_uint(a.w) & wrp::kPatchFlag) {
+                float lo[3], hi[3];
+                wrp::load_patch_box(patches, i, lo, hi);
+                if (box_entry(r, lo[0], hi[0], lo[1], hi[1], lo[2], hi[2], tmin, t) != __int_as_float(0x7f800000)) ps.pend = i;
+                continue;
+            }
+            const float4 b = __ldg(tris + 3 * i + 1);
+            const float4 c = __ldg(tris + 3 * i + 2);
+            float th, uh, vh;
+            if (tri_test(r, a, b, c, tmin, t, th, uh, vh) && (any_hit || th < t || tri == MISS)) {
+                t = th;
+                tri = i;
+                bu = uh;
+                bv = vh;
+                found = any_hit;
+            }
+        }
+        const uint32_t active = __activemask();
+        const bool waits = !found && ps.pend != MISS;
+        const uint32_t waiting = __ballot_sync(active, waits);
+        const uint32_t others = __ballot_sync(active, !waits && !found && (node != kTraceDone || leaf < 0 || ps.cur < ps.end));
+        if (waits && (__popc(waiting) >= kPatchWait || others == 0u)) {
+            const uint32_t i = ps.pend;
+            ps.pend = MISS;
+            const float4 a = __ldg(tris + 3 * i), b = __ldg(tris + 3 * i + 1), c = __ldg(tris + 3 * i + 2);
+            if (patch_test(pr, patches, i, a, b, c, tmin, t, bu, bv)) {
+                tri = i;
+                found = any_hit;
+            }
+        }
+        if (found) {
+            node = kTraceDone;
+            leaf = 0;
+            ps = PatchState{0u, 0u, MISS};
+            return true;
+        }
+        if ((node != kTraceDone || leaf < 0 || ps.cur < ps.end || ps.pend != MISS) && __popc(__activemask()) < min_active)
+            return false;
+    }
+    return true;
+}
+
 // one whole query (the k_trace_batch path)
 template <bool ANY_HIT, bool PHONG, bool COUNT>
 __device__ __forceinline__ bool traverse(const float4 *__restrict__ nodes, const float4 *__restrict__ tris, f3 o,
@@ -281,8 +370,12 @@ __device__ __forceinline__ bool traverse(const float4 *__restrict__ nodes, const
     tri = MISS;
     t = tmax;
     st.clear();
-    traverse_steps<ANY_HIT, PHONG, !ANY_HIT, COUNT>(nodes, tris, r, tmin, t, tri, bu, bv, node, leaf, st, nv, nt, 0, patches,
-                                               pr);
+    if (PHONG) {
+        PatchState ps{0u, 0u, MISS};
+        traverse_patches<COUNT>(nodes, tris, patches, r, pr, ANY_HIT, tmin, t, tri, bu, bv, node, leaf, ps, st, nv, nt, 0);
+    } else {
+        traverse_steps<ANY_HIT, !ANY_HIT, COUNT>(nodes, tris, r, tmin, t, tri, bu, bv, node, leaf, st, nv, nt, 0);
+    }
     return tri != MISS;
 }
 
