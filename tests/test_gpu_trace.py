@@ -316,3 +316,48 @@ def test_long_batches_answer_like_short_ones(wr_lib, name, n):
         many = sc.trace_closest(rays[take]) + sc.trace_hits(rays[take])[3:] + (sc.trace_occluded(rays[take]),)
     for a, b in zip(few, many):
         assert np.array_equal(a[take], b)
+
+
+@pytest.mark.parametrize("scale", [1.0, 1e3])
+@pytest.mark.parametrize("bend", [0.0, 0.05, 0.6, 1.2])
+def test_patch_culling_keeps_every_hit(wr_lib, oracle_lib, tmp_path, bend, scale):
+    """Patches from flat to strongly curved, fat and thin, at small and large scales: the planes that
+    a ray must meet before the FP64 test keep every hit of the oracle, which has no such planes."""
+    from wurstrenderer_b200 import scenes
+    rng = np.random.default_rng(int(100 * bend) + 7)
+    base, smooth = scenes.SceneSpec(), scenes.SceneSpec()
+    s = np.float32(scale)
+    p, t = scenes.quad((5.0, 9.0, 5.0), (6.0, 9.0, 5.0), (6.0, 9.0, 6.0), (5.0, 9.0, 6.0))
+    base.add("light", scenes.Material("m_light", ke=(5.0, 5.0, 5.0)), p * s, t)
+    grey = scenes.Material("m_grey", kd=(0.5, 0.5, 0.5))
+    centres = rng.uniform(-1.5, 1.5, (60, 3))
+    for i, c in enumerate(centres):
+        tri = c + rng.normal(size=(3, 3)) * 0.4
+        if i % 4 == 0:                       # a thin one
+            tri[2] = tri[0] + 0.5 * (tri[1] - tri[0]) + 0.02 * rng.normal(size=3)
+        g = np.cross(tri[1] - tri[0], tri[2] - tri[0])
+        n = g / np.linalg.norm(g) + bend * rng.normal(size=(3, 3))
+        n /= np.linalg.norm(n, axis=1, keepdims=True)
+        smooth.add("p%02d" % i, grey, (tri * scale).astype(np.float32), np.array([[0, 1, 2]]), normals=n.astype(np.float32))
+    cam = {"pos": [0.0, 0.0, 4.0 * scale], "lookat": [0.0, 0.0, 0.0], "up": [0.0, 1.0, 0.0], "fovy": 60.0,
+           "resolution": [16, 16]}
+    path = scenes.write_scene_entries(str(tmp_path), "patches", [("base", base, None),
+                                                                ("smooth", smooth, {"phong_tessellation": True})],
+                                      cam, [scenes.nee_render("patches.pfm", 1, 3)])
+    m = 6000
+    rays = np.zeros((m, 8), np.float32)
+    o = rng.normal(size=(m, 3)) * 3.0
+    d = centres[rng.integers(0, len(centres), m)] + 0.35 * rng.normal(size=(m, 3)) - o
+    rays[:, 0:3] = o * scale
+    rays[:, 4:7] = d / np.linalg.norm(d, axis=1, keepdims=True)
+    rays[:, 3], rays[:, 7] = 1e-4 * scale, np.inf
+    g_o, p_o, t_o, _ = oracle_lib.OracleScene(path).trace_closest(rays)
+    with wr_lib.Scene.from_file(path) as sc:
+        g, p, t, _ = sc.trace_closest(rays)
+        occ = sc.trace_occluded(rays)
+    same = (g == g_o) & (p == p_o)
+    with np.errstate(invalid="ignore"):
+        tie = np.abs(t_o - t) <= 1e-5 * np.maximum(np.abs(t_o), 1.0)
+    assert (~same & ~tie).sum() == 0, "mismatching rays: %s" % np.nonzero(~same & ~tie)[0][:10]
+    assert (g_o >= 0).mean() > 0.1 or bend == 0.0
+    assert np.array_equal(occ != 0, g >= 0)

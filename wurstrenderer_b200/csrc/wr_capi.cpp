@@ -143,11 +143,13 @@ void build_device_scene(wr_scene &s) {
     // Phong tessellation patches: FP64 unit normals and boxes per patch (global order)
     std::vector<uint8_t> is_patch(ntri, 0);
     std::vector<double> patch_n;          // 9 per triangle (only patches are filled)
+    std::vector<float> patch_planes;      // 20 per triangle: wrp::patch_hull
     std::vector<float> box_near, box_out; // 6 per triangle: the bound rounded to nearest / outward
     uint32_t npatch = 0;
     for (const wr::Mesh &m : h.meshes) if (m.phong) npatch += m.num_triangles();
     if (npatch) {
         patch_n.assign(size_t(ntri) * 9, 0.0);
+        patch_planes.assign(size_t(ntri) * 20, 0.f);
         box_near.assign(size_t(ntri) * 6, 0.f);
         box_out.assign(size_t(ntri) * 6, 0.f);
     }
@@ -184,6 +186,7 @@ void build_device_scene(wr_scene &s) {
                 }
                 double lo[3], hi[3];
                 wrp::patch_bound(P, lo, hi);
+                wrp::patch_hull(P, &patch_planes[20 * g]);
                 for (int k = 0; k < 3; ++k) {
                     // Embree keeps float(bound) (embreeaccel.h:63-75); the BVH uses the box
                     // rounded outward so that it contains the FP64 bound
@@ -289,10 +292,11 @@ void build_device_scene(wr_scene &s) {
         memcpy(&o[7], &tri_mesh[g], 4);
         memcpy(&o[11], &tri_prim[g], 4);
         leaf_mat[i] = tri_code[g];
-        if (is_patch[g]) {   // n1 n2 n3, then the outward box as 6 floats in the last 3 doubles
+        if (is_patch[g]) {   // n1 n2 n3, the outward box as 6 floats, the hull planes as 20
             double *pd = &patchd[size_t(wrp::kPatchDoubles) * i];
             for (int k = 0; k < 9; ++k) pd[k] = patch_n[9 * size_t(g) + k];
             memcpy(pd + 9, &box_out[6 * size_t(g)], 24);
+            memcpy(pd + wrp::kHullDouble, &patch_planes[20 * size_t(g)], 80);
         }
     }
     if (wide) upload(s.wnodes, wbvh.nodes, st);

@@ -135,13 +135,14 @@ __device__ __forceinline__ bool patch_test(const PatchRay &pr, const double *pat
     return true;
 }
 
-// leaf primitive i is a patch: its own box, then the FP64 test
+// leaf primitive i is a patch: its own box and hull planes, then the FP64 test
 __device__ __forceinline__ bool patch_leaf_test(const RayPre &r, const PatchRay &pr, const double *patches, uint32_t i,
                                                 float4 a, float4 b, float4 c, float tmin, float &t, float &bu,
                                                 float &bv) {
     float lo[3], hi[3];
     wrp::load_patch_box(patches, i, lo, hi);
     if (box_entry(r, lo[0], hi[0], lo[1], hi[1], lo[2], hi[2], tmin, t) == __int_as_float(0x7f800000)) return false;
+    if (!wrp::meets_hull(patches, i, make_float3(a.x, a.y, a.z), pr.ox, pr.oy, pr.oz, pr.dx, pr.dy, pr.dz, tmin, t)) return false;
     return patch_test(pr, patches, i, a, b, c, tmin, t, bu, bv);
 }
 
@@ -270,7 +271,8 @@ __device__ __forceinline__ bool traverse_steps(const float4 *__restrict__ nodes,
 // different places in it thrashed the instruction cache. Here a lane whose patch passes its own box
 // holds it (`pend`) and waits, descending further where it can, until kPatchWait lanes of the warp hold
 // one or none can do anything else: 27.0 -> 18.9 ms for a frame of 56,000 patches (kPatchWait 1 / 8 / 12 /
-// 16 / 20: 19.6 / 18.7 / 18.9 / 18.8 / 19.0), 16.9 with the registers that the fused kernel then gives it.
+// 16 / 20: 19.6 / 18.7 / 18.9 / 18.8 / 19.0). A patch also has to pass its hull planes (meets_hull): 10 FP64
+// tests per closest-hit ray of that frame became 1.65, with 0.47 hits, and 16.9 ms 14.7.
 // The postponed leaf's remaining primitives are [cur, end).
 constexpr int kPatchWait = 12;
 
@@ -320,7 +322,9 @@ __device__ __forceinline__ bool traverse_patches(const float4 *__restrict__ node
             if (__float_as_uint(a.w) & wrp::kPatchFlag) {
                 float lo[3], hi[3];
                 wrp::load_patch_box(patches, i, lo, hi);
-                if (box_entry(r, lo[0], hi[0], lo[1], hi[1], lo[2], hi[2], tmin, t) != __int_as_float(0x7f800000)) ps.pend = i;
+                if (box_entry(r, lo[0], hi[0], lo[1], hi[1], lo[2], hi[2], tmin, t) != __int_as_float(0x7f800000) &&
+                    wrp::meets_hull(patches, i, make_float3(a.x, a.y, a.z), pr.ox, pr.oy, pr.oz, pr.dx, pr.dy, pr.dz, tmin, t))
+                    ps.pend = i;
                 continue;
             }
             const float4 b = __ldg(tris + 3 * i + 1);
