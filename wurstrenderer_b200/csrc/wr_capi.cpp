@@ -589,6 +589,14 @@ void render_jobs(wr_scene &s, const std::vector<HostJob> &jobs, const wr_render_
     // 41.6 ms for the 1.16M-triangle frame, 95.5 / 93.3 / 90.6 / 98.8 for 24 Cornell jobs.
     uint32_t capacity = desc.queue_capacity > 0 ? uint32_t(desc.queue_capacity) : (1u << 22);
     capacity = uint32_t(std::min<unsigned long long>(capacity, std::max<unsigned long long>(total, 1024ull)));
+    // A render whose samples all fit the wavefront takes max_nverts - 1 bounce iterations and no
+    // more: they are launched one after another with nothing to decide in between, each kernel's
+    // set-up overlapping the one before it. Building and instantiating a graph costs the host more
+    // than these few launches, and the overlap shortens the device's part (64x48 Cornell preview:
+    // 0.50 ms by graph, 0.35 by plain launches, 0.27 by overlapping ones; 256x256 at 16 spp 1.55,
+    // 1.31, 1.24). Longer renders, whose number of iterations only the device knows, are one graph;
+    // overlapping the launches inside it changes nothing (44.0 against 43.9 ms for the 1M frame).
+    const bool one_wave = total <= capacity && max_nverts <= 64;
     ensure_wave(s, capacity, total_pix);
     cudaStream_t st = s.stream;
 
@@ -625,7 +633,10 @@ void render_jobs(wr_scene &s, const std::vector<HostJob> &jobs, const wr_render_
     r.guide_sms = sms;
     if (desc.fetch_threshold < 0 || desc.fetch_threshold > 32)
         throw Error(WR_ERR_INVALID_ARGUMENT, "fetch_threshold must be 0..32");
-    r.fetch_min = desc.fetch_threshold > 0 ? desc.fetch_threshold : 20;
+    // lanes still traversing below which a warp takes new rays: 8 / 12 / 16 / 20 / 24 measured 41.9 / 41.8 /
+    // 41.9 / 42.3 / 43.1 ms for the 1.16M-triangle frame, but 12 / 20 / 24 14.1 / 13.9 / 14.0 for 56,000
+    // patches, where the refill interrupts gathered patch tests
+    r.fetch_min = desc.fetch_threshold > 0 ? desc.fetch_threshold : s.dev.patches ? 20 : 12;
     r.num_jobs = int(table.size());
     r.job0 = table[0];
     r.nee_only = 1;
@@ -666,14 +677,6 @@ void render_jobs(wr_scene &s, const std::vector<HostJob> &jobs, const wr_render_
         WR_CUDA(cudaMemsetAsync(b.sample_next, 0, 8, st));
     };
     const bool trace = max_nverts > 1;
-    // A render whose samples all fit the wavefront takes max_nverts - 1 bounce iterations and no
-    // more: they are launched one after another with nothing to decide in between, each kernel's
-    // set-up overlapping the one before it. Building and instantiating a graph costs the host more
-    // than these few launches, and the overlap shortens the device's part (64x48 Cornell preview:
-    // 0.50 ms by graph, 0.35 by plain launches, 0.27 by overlapping ones; 256x256 at 16 spp 1.55,
-    // 1.31, 1.24). Longer renders, whose number of iterations only the device knows, are one graph;
-    // overlapping the launches inside it changes nothing (44.0 against 43.9 ms for the 1M frame).
-    const bool one_wave = total <= capacity && max_nverts <= 64;
     if (profile) {
         // one kernel at a time, bracketed by events, to attribute device time per kernel
         WR_CUDA(cudaMemsetAsync(s.w_prof.p, 0, 16 * 8, st));
