@@ -142,19 +142,20 @@ void build_device_scene(wr_scene &s) {
     std::vector<uint32_t> tri_mesh(ntri), tri_prim(ntri), tri_code(ntri);
     // Phong tessellation patches: FP64 unit normals and boxes per patch (global order)
     std::vector<uint8_t> is_patch(ntri, 0);
-    std::vector<double> patch_n;          // 9 per triangle (only patches are filled)
-    std::vector<float> patch_planes;      // 20 per triangle: wrp::patch_hull
+    std::vector<double> patchd;           // device records, one per patch (wrp::kPatchDoubles)
+    std::vector<uint32_t> patch_of;       // a patch triangle's record
     std::vector<float> box_near, box_out; // 6 per triangle: the bound rounded to nearest / outward
     uint32_t npatch = 0;
     for (const wr::Mesh &m : h.meshes) if (m.phong) npatch += m.num_triangles();
     if (npatch) {
-        patch_n.assign(size_t(ntri) * 9, 0.0);
-        patch_planes.assign(size_t(ntri) * 20, 0.f);
+        patchd.assign(size_t(npatch) * wrp::kPatchDoubles, 0.0);
+        patch_of.assign(ntri, 0u);
         box_near.assign(size_t(ntri) * 6, 0.f);
         box_out.assign(size_t(ntri) * 6, 0.f);
     }
     {
         size_t g = 0;
+        uint32_t next_patch = 0;
         for (size_t mi = 0; mi < h.meshes.size(); ++mi) {
             const wr::Mesh &m = h.meshes[mi];
             const uint32_t code = m.light >= 0 ? (wrd::LIGHT_BIT | uint32_t(m.light)) : uint32_t(m.material);
@@ -173,6 +174,7 @@ void build_device_scene(wr_scene &s) {
                 // the PhongMeshGeometry of this triangle: normals as AssimpInOut stores them
                 // (zero when of ~zero length, else normalised in FP64; assimpio.h:211-223)
                 wrp::Patch<double> P;
+                double *const pd = &patchd[size_t(wrp::kPatchDoubles) * next_patch];
                 for (int c = 0; c < 3; ++c) {
                     const uint32_t vi = m.indices[3 * t + c];
                     const float *q = &m.positions[3 * size_t(vi)];
@@ -180,13 +182,15 @@ void build_device_scene(wr_scene &s) {
                     P.p[c] = wrp::v3<double>(q[0], q[1], q[2]);
                     const wrp::V<double> n = wrp::v3<double>(nn[0], nn[1], nn[2]);
                     P.n[c] = wrp::is_approx_zero(wrp::length(n)) ? wrp::v3<double>(0.0, 0.0, 0.0) : wrp::normalize(n);
-                    patch_n[9 * g + 3 * c + 0] = P.n[c].x;
-                    patch_n[9 * g + 3 * c + 1] = P.n[c].y;
-                    patch_n[9 * g + 3 * c + 2] = P.n[c].z;
+                    pd[3 * c + 0] = P.n[c].x;
+                    pd[3 * c + 1] = P.n[c].y;
+                    pd[3 * c + 2] = P.n[c].z;
                 }
                 double lo[3], hi[3];
                 wrp::patch_bound(P, lo, hi);
-                wrp::patch_hull(P, &patch_planes[20 * g]);
+                float planes[20];
+                wrp::patch_hull(P, planes);
+                memcpy(pd + wrp::kHullDouble, planes, 80);
                 for (int k = 0; k < 3; ++k) {
                     // Embree keeps float(bound) (embreeaccel.h:63-75); the BVH uses the box
                     // rounded outward so that it contains the FP64 bound
@@ -198,7 +202,9 @@ void build_device_scene(wr_scene &s) {
                     box_out[6 * g + k] = fl;
                     box_out[6 * g + 3 + k] = fh;
                 }
+                memcpy(pd + 9, &box_out[6 * g], 24);
                 is_patch[g] = 1;
+                patch_of[g] = next_patch++;
             }
         }
     }
@@ -281,23 +287,16 @@ void build_device_scene(wr_scene &s) {
     if (bvh.depth > wrd::kMaxStack) throw Error(WR_ERR_UNSUPPORTED, "BVH deeper than the traversal stack");
     std::vector<float> trisf(size_t(ntri) * 12);
     std::vector<uint32_t> leaf_mat(ntri);
-    std::vector<double> patchd(npatch ? size_t(ntri) * wrp::kPatchDoubles : 0, 0.0);
     for (uint32_t i = 0; i < ntri; ++i) {
         const uint32_t g = bvh.tri_order[i];
         float *o = &trisf[12 * size_t(i)];
         for (int c = 0; c < 3; ++c)
             for (int k = 0; k < 3; ++k) o[4 * c + k] = verts[9 * size_t(g) + 3 * c + k];
-        const uint32_t gw = g | (is_patch[g] ? wrp::kPatchFlag : 0u);
+        const uint32_t gw = is_patch[g] ? patch_of[g] | wrp::kPatchFlag : g;   // a patch: its record
         memcpy(&o[3], &gw, 4);
         memcpy(&o[7], &tri_mesh[g], 4);
         memcpy(&o[11], &tri_prim[g], 4);
         leaf_mat[i] = tri_code[g];
-        if (is_patch[g]) {   // n1 n2 n3, the outward box as 6 floats, the hull planes as 20
-            double *pd = &patchd[size_t(wrp::kPatchDoubles) * i];
-            for (int k = 0; k < 9; ++k) pd[k] = patch_n[9 * size_t(g) + k];
-            memcpy(pd + 9, &box_out[6 * size_t(g)], 24);
-            memcpy(pd + wrp::kHullDouble, &patch_planes[20 * size_t(g)], 80);
-        }
     }
     if (wide) upload(s.wnodes, wbvh.nodes, st);
     else upload(s.nodes, bvh.nodes, st);

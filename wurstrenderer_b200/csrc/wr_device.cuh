@@ -2,7 +2,8 @@
 //
 // Scene data in HBM (all 16-byte aligned, read through the non-coherent path):
 //   nodes      4 x float4 per binary BVH node (layout in wr_bvh.cpp)
-//   tris       3 x float4 per triangle in leaf order: v0.xyz|global id, v1.xyz|mesh id, v2.xyz|prim id
+//   tris       3 x float4 per triangle in leaf order: v0.xyz|global id (a patch: flag and record), v1.xyz|mesh id,
+//              v2.xyz|prim id
 //   tri_mat    uint32 per leaf-order triangle: material index, or LIGHT_BIT | light index
 //   materials  DevMaterial per surface material
 //   lights     DevLight per area light, light_tris 3 x float4 per emitter triangle
@@ -95,7 +96,7 @@ struct DevScene {
     const float4 *nodes;            // binary BVH (4 x float4 per node)
     const uint4 *wnodes;            // compressed 8-wide BVH (5 x uint4 per node), nullptr when binary
     const float4 *tris;             // leaf order: p0, p1, p2 (.w: index | patch flag, mesh, primitive)
-    const double *patches;          // Phong tessellation patches (wrp::kPatchDoubles per leaf primitive),
+    const double *patches;          // Phong tessellation patches (wrp::kPatchDoubles per patch),
                                     // nullptr when the scene has none
     int stack_words;                // traversal stack entries per thread (the tree's depth and the sentinel)
     const uint32_t *tri_mat;

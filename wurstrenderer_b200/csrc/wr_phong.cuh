@@ -491,8 +491,7 @@ __device__ __forceinline__ float3 oct_decode(float px, float py) {
     return make_float3(x * inv, y * inv, z * inv);
 }
 
-// the patch of leaf primitive `i`: positions from its float leaf record, normals (FP64) from
-// the patch array
+// the patch of record `i`: positions from its float leaf record, normals (FP64) from the patch array
 __device__ __forceinline__ Patch<Rd> load_patch(const double *patches, uint32_t i, float4 a, float4 b, float4 c) {
     const double2 *q = reinterpret_cast<const double2 *>(patches + size_t(kPatchDoubles) * i);
     const double2 n01 = __ldg(q + 0), n23 = __ldg(q + 1), n45 = __ldg(q + 2), n67 = __ldg(q + 3), n8x = __ldg(q + 4);

@@ -120,11 +120,14 @@ struct PatchRay {
     float ox, oy, oz, dx, dy, dz;
 };
 
-// the FP64 test of patch i, whose own box the ray has passed, against (tmin, t]; on a hit lowers t and
-// stores the encoded normal in (bu, bv)
-__device__ __forceinline__ bool patch_test(const PatchRay &pr, const double *patches, uint32_t i, float4 a, float4 b,
+// a patch primitive's record
+__device__ __forceinline__ uint32_t patch_record(float4 a) { return __float_as_uint(a.w) & ~wrp::kPatchFlag; }
+
+// the FP64 test of the patch (a, b, c), whose own box the ray has passed, against (tmin, t]; on a hit
+// lowers t and stores the encoded normal in (bu, bv)
+__device__ __forceinline__ bool patch_test(const PatchRay &pr, const double *patches, float4 a, float4 b,
                                            float4 c, float tmin, float &t, float &bu, float &bv) {
-    const wrp::Patch<wrp::Rd> P = wrp::load_patch(patches, i, a, b, c);
+    const wrp::Patch<wrp::Rd> P = wrp::load_patch(patches, patch_record(a), a, b, c);
     wrp::Rd tm = wrp::Rd(double(t));
     wrp::V<wrp::Rd> n;
     if (!wrp::patch_intersect(P, pr.ox, pr.oy, pr.oz, pr.dx, pr.dy, pr.dz, tmin, tm, n)) return false;
@@ -135,15 +138,16 @@ __device__ __forceinline__ bool patch_test(const PatchRay &pr, const double *pat
     return true;
 }
 
-// leaf primitive i is a patch: its own box and hull planes, then the FP64 test
-__device__ __forceinline__ bool patch_leaf_test(const RayPre &r, const PatchRay &pr, const double *patches, uint32_t i,
-                                                float4 a, float4 b, float4 c, float tmin, float &t, float &bu,
+// a leaf's patch: its own box and hull planes, then the FP64 test
+__device__ __forceinline__ bool patch_leaf_test(const RayPre &r, const PatchRay &pr, const double *patches, float4 a,
+                                                float4 b, float4 c, float tmin, float &t, float &bu,
                                                 float &bv) {
+    const uint32_t i = patch_record(a);
     float lo[3], hi[3];
     wrp::load_patch_box(patches, i, lo, hi);
     if (box_entry(r, lo[0], hi[0], lo[1], hi[1], lo[2], hi[2], tmin, t) == __int_as_float(0x7f800000)) return false;
     if (!wrp::meets_hull(patches, i, make_float3(a.x, a.y, a.z), pr.ox, pr.oy, pr.oz, pr.dx, pr.dy, pr.dz, tmin, t)) return false;
-    return patch_test(pr, patches, i, a, b, c, tmin, t, bu, bv);
+    return patch_test(pr, patches, a, b, c, tmin, t, bu, bv);
 }
 
 // unit geometry normal of a hit on leaf primitive (a, b, c): the triangle's face normal,
@@ -321,9 +325,10 @@ __device__ __forceinline__ bool traverse_patches(const float4 *__restrict__ node
             if (COUNT) ++nt;
             if (__float_as_uint(a.w) & wrp::kPatchFlag) {
                 float lo[3], hi[3];
-                wrp::load_patch_box(patches, i, lo, hi);
+                const uint32_t rec = patch_record(a);
+                wrp::load_patch_box(patches, rec, lo, hi);
                 if (box_entry(r, lo[0], hi[0], lo[1], hi[1], lo[2], hi[2], tmin, t) != __int_as_float(0x7f800000) &&
-                    wrp::meets_hull(patches, i, make_float3(a.x, a.y, a.z), pr.ox, pr.oy, pr.oz, pr.dx, pr.dy, pr.dz, tmin, t))
+                    wrp::meets_hull(patches, rec, make_float3(a.x, a.y, a.z), pr.ox, pr.oy, pr.oz, pr.dx, pr.dy, pr.dz, tmin, t))
                     ps.pend = i;
                 continue;
             }
@@ -346,7 +351,7 @@ __device__ __forceinline__ bool traverse_patches(const float4 *__restrict__ node
             const uint32_t i = ps.pend;
             ps.pend = MISS;
             const float4 a = __ldg(tris + 3 * i), b = __ldg(tris + 3 * i + 1), c = __ldg(tris + 3 * i + 2);
-            if (patch_test(pr, patches, i, a, b, c, tmin, t, bu, bv)) {
+            if (patch_test(pr, patches, a, b, c, tmin, t, bu, bv)) {
                 tri = i;
                 found = any_hit;
             }
@@ -467,7 +472,7 @@ __device__ __forceinline__ bool traverse_steps_w8(const uint4 *__restrict__ wnod
                 const float4 c = __ldg(tris + 3 * i + 2);
                 if (COUNT) ++nt;
                 if (PHONG && (__float_as_uint(a.w) & wrp::kPatchFlag)) {
-                    if (patch_leaf_test(r, pr, patches, i, a, b, c, tmin, t, bu, bv)) {
+                    if (patch_leaf_test(r, pr, patches, a, b, c, tmin, t, bu, bv)) {
                         tri = i;
                         if (ANY_HIT) {
                             ws.node = -1;
