@@ -188,9 +188,6 @@ void build_device_scene(wr_scene &s) {
                 }
                 double lo[3], hi[3];
                 wrp::patch_bound(P, lo, hi);
-                float planes[20];
-                wrp::patch_hull(P, planes);
-                memcpy(pd + wrp::kHullDouble, planes, 80);
                 for (int k = 0; k < 3; ++k) {
                     // Embree keeps float(bound) (embreeaccel.h:63-75); the BVH uses the box
                     // rounded outward so that it contains the FP64 bound

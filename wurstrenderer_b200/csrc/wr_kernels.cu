@@ -993,11 +993,11 @@ __global__ void __launch_bounds__(BLOCK) k_trace_pair(DevScene s, WaveArgs w) {
     trace_pair<BLOCK, false, WIDE, COUNT>(s, w);
 }
 
-// The FP64 patch test wants 222 registers (256 resident threads per SM). Since most of a launch is
-// traversal, more threads with a test that spills a little are the better side: 256 / 384 / 512 / 640 /
-// 768 threads per SM take 14.7 / 13.9 / 14.1 / 14.6 / 15.1 ms for a frame of 56,000 patches.
+// The FP64 patch test wants 222 registers, which leaves 256 resident threads per SM. Held to 168
+// registers (384 threads) it spills and takes 18.7 ms for a frame of 56,000 patches that takes 16.9
+// with all its registers; with 128 threads per SM it takes 25.4.
 template <int BLOCK, bool WIDE, bool COUNT>
-__global__ void __launch_bounds__(BLOCK, 384 / BLOCK) k_trace_pair_phong(DevScene s, WaveArgs w) {
+__global__ void __launch_bounds__(BLOCK, 256 / BLOCK) k_trace_pair_phong(DevScene s, WaveArgs w) {
     trace_pair<BLOCK, true, WIDE, COUNT>(s, w);
 }
 

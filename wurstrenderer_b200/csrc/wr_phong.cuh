@@ -42,9 +42,7 @@
 namespace wrp {
 
 constexpr uint32_t kPatchFlag = 0x80000000u;   // set in the leaf record's first .w word
-// a patch's record: n1 n2 n3 (9 doubles), float box lo/hi (6 floats), hull planes (5 x 4 floats)
-constexpr int kPatchDoubles = 22;
-constexpr int kHullDouble = 12;                 // the hull planes' first double
+constexpr int kPatchDoubles = 12;               // n1 n2 n3 (9 doubles) + float box lo/hi (6 floats)
 constexpr double kAlpha = 3.0 / 4.0;
 constexpr double kPi = 3.141592653589793238462643383279502884197169399375105820974;
 constexpr double kSmall = 1e-12;                // Math::SmallValue
@@ -271,60 +269,6 @@ inline void patch_bound(const Patch<double> &P, double lo[3], double hi[3]) {
     }
 }
 
-// Five planes around a patch, for a cheap float test before the FP64 one. With barycentric weights w_i
-// the surface is sum_ij w_i w_j ((1 - alpha) p_j + alpha pi_i(p_j)), pi_i the projection onto vertex i's
-// tangent plane: a quadratic Bezier triangle whose control points are the vertices and, per edge, the
-// mean of the two mixed terms, so it lies in the hull of those six points. hull[0] = (g, -min), hull[4].x
-// = max of g . (x - p1) over them for the unit face normal g; hull[1..3] = (m_e, max of m_e . (x - p1))
-// for the outward edge normals m_e in the triangle's plane; all maxima raised by 1e-4 of the patch's
-// size. A triangle without an area, and a patch that
-// the FP64 test's own thresholds blur, get planes that keep every ray.
-inline void patch_hull(const Patch<double> &P, float hull[20]) {
-    for (int i = 0; i < 20; ++i) hull[i] = 0.f;
-    for (int i : {3, 7, 11, 15, 16}) hull[i] = std::numeric_limits<float>::infinity();
-    V<double> b[6];
-    double size = 0.0;
-    for (int i = 0; i < 3; ++i) {
-        const int j = (i + 1) % 3;
-        auto onto = [&](int t, int of) { return P.p[of] - dot(P.p[of] - P.p[t], P.n[t]) * P.n[t]; };
-        b[i] = P.p[i];
-        b[3 + i] = (1.0 - kAlpha) * 0.5 * (P.p[i] + P.p[j]) + kAlpha * 0.5 * (onto(i, j) + onto(j, i));
-    }
-    for (int i = 1; i < 6; ++i) size = tmax_(size, length(b[i] - P.p[0]));
-    const V<double> c = cross(P.p[1] - P.p[0], P.p[2] - P.p[0]);
-    const double area = length(c);
-    if (!(area > 1e-6 * size * size) || !(size < 1e30)) return;   // a sliver, or not finite
-    // The test's solvers take a leading coefficient below 1e-12 for zero. For a patch whose coefficients
-    // are of that order (a3 of eq. 16 is about curvature x size^2 / 4) they find points off the ray, and
-    // those hits belong to the answer: such a patch keeps every ray. At 10^6 times that order the dropped
-    // term moves a hit by 1e-6 of the patch's size, well inside the planes' margin.
-    const Coeffs<double> k = coeffs(P);
-    const double curvature = tmax_(length(k.c12), tmax_(length(k.c23), length(k.c31)));
-    if (!(curvature * size * size > 4e-6)) return;
-    const V<double> g = c * (1.0 / area);
-    double lo = 0.0, hi = 0.0;
-    for (int i = 1; i < 6; ++i) {
-        const double h = dot(g, b[i] - P.p[0]);
-        lo = h < lo ? h : lo;
-        hi = h > hi ? h : hi;
-    }
-    const double more = 1e-4 * size;
-    auto put = [&](int k, const V<double> &n, double d) {
-        hull[4 * k] = float(n.x);
-        hull[4 * k + 1] = float(n.y);
-        hull[4 * k + 2] = float(n.z);
-        hull[4 * k + 3] = float(d);
-    };
-    put(0, g, -lo + more);
-    hull[16] = float(hi + more);
-    for (int e = 0; e < 3; ++e) {
-        const V<double> m = normalize(cross(P.p[(e + 1) % 3] - P.p[e], g));
-        double d = dot(m, P.p[e] - P.p[0]);
-        for (int i = 0; i < 6; ++i) d = tmax_(d, dot(m, b[i] - P.p[0]));
-        put(1 + e, m, d + more);
-    }
-}
-
 // PhongMeshGeometry::intersect (phongmesh.h:178-368) for a float ray as Embree passes it
 // (embreeaccel.h:77-99). Accepts a candidate with tmin <= t <= tmax, lowering tmax each
 // time, and returns whether any was accepted; `normal` is the unit patch normal there.
@@ -511,36 +455,6 @@ __device__ __forceinline__ void load_patch_box(const double *patches, uint32_t i
     const float2 a = __ldg(q), b = __ldg(q + 1), c = __ldg(q + 2);
     lo[0] = a.x; lo[1] = a.y; lo[2] = b.x;
     hi[0] = b.y; hi[1] = c.x; hi[2] = c.y;
-}
-
-// Whether the float ray (o, d) on [tmin, tmax] meets patch i's hull planes; p0 is its first vertex. The
-// planes are moved out by 1e-5 of the distances involved, some forty times what the float
-// arithmetic can be off, so a ray that meets the patch passes; a NaN passes too.
-__device__ __forceinline__ bool meets_hull(const double *patches, uint32_t i, float3 p0, float ox, float oy, float oz,
-                                           float dx, float dy, float dz, float tmin, float tmax) {
-    const float4 *h = reinterpret_cast<const float4 *>(patches + size_t(kPatchDoubles) * i + kHullDouble);
-    const float qx = ox - p0.x, qy = oy - p0.y, qz = oz - p0.z;
-    const float more = 1e-5f * (fabsf(qx) + fabsf(qy) + fabsf(qz)) +
-                       1e-6f * (fabsf(ox) + fabsf(oy) + fabsf(oz) + fabsf(p0.x) + fabsf(p0.y) + fabsf(p0.z));
-    float tn = tmin, tf = tmax;
-    bool out = false;
-    auto clip = [&](float s0, float s1, float c) {   // keep s0 + t s1 <= c + more
-        const float r = c + more - s0;
-        const float t = r / s1;
-        if (s1 > 0.f) tf = fminf(tf, t);
-        else if (s1 < 0.f) tn = fmaxf(tn, t);
-        else out = out || r < 0.f;
-    };
-    const float4 g = __ldg(h);
-    const float s0 = g.x * qx + g.y * qy + g.z * qz, s1 = g.x * dx + g.y * dy + g.z * dz;
-    clip(-s0, -s1, g.w);
-    clip(s0, s1, __ldg(reinterpret_cast<const float *>(h + 4)));
-#pragma unroll
-    for (int e = 1; e < 4; ++e) {
-        const float4 m = __ldg(h + e);
-        clip(m.x * qx + m.y * qy + m.z * qz, m.x * dx + m.y * dy + m.z * dz, m.w);
-    }
-    return !(out || tn > tf);
 }
 #endif
 

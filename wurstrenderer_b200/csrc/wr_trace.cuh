@@ -138,15 +138,13 @@ __device__ __forceinline__ bool patch_test(const PatchRay &pr, const double *pat
     return true;
 }
 
-// a leaf's patch: its own box and hull planes, then the FP64 test
+// a leaf's patch: its own box, then the FP64 test
 __device__ __forceinline__ bool patch_leaf_test(const RayPre &r, const PatchRay &pr, const double *patches, float4 a,
                                                 float4 b, float4 c, float tmin, float &t, float &bu,
                                                 float &bv) {
-    const uint32_t i = patch_record(a);
     float lo[3], hi[3];
-    wrp::load_patch_box(patches, i, lo, hi);
+    wrp::load_patch_box(patches, patch_record(a), lo, hi);
     if (box_entry(r, lo[0], hi[0], lo[1], hi[1], lo[2], hi[2], tmin, t) == __int_as_float(0x7f800000)) return false;
-    if (!wrp::meets_hull(patches, i, make_float3(a.x, a.y, a.z), pr.ox, pr.oy, pr.oz, pr.dx, pr.dy, pr.dz, tmin, t)) return false;
     return patch_test(pr, patches, a, b, c, tmin, t, bu, bv);
 }
 
@@ -275,8 +273,11 @@ __device__ __forceinline__ bool traverse_steps(const float4 *__restrict__ nodes,
 // different places in it thrashed the instruction cache. Here a lane whose patch passes its own box
 // holds it (`pend`) and waits, descending further where it can, until kPatchWait lanes of the warp hold
 // one or none can do anything else: 27.0 -> 18.9 ms for a frame of 56,000 patches (kPatchWait 1 / 8 / 12 /
-// 16 / 20: 19.6 / 18.7 / 18.9 / 18.8 / 19.0). A patch also has to pass its hull planes (meets_hull): 10 FP64
-// tests per closest-hit ray of that frame became 1.65, with 0.47 hits, and 16.9 ms 14.7.
+// 16 / 20: 19.6 / 18.7 / 18.9 / 18.8 / 19.0), 16.9 with the registers that the fused kernel then gives it.
+// Nothing but its own box may keep a ray from a patch's FP64 test: the test also accepts points off the
+// ray, and they are part of the answer. Where two vertex normals equal the face normal, or on a cylinder,
+// the pencil of conics degenerates and a third of all accepted points lie outside the patch's convex
+// hull widened by 1e-4 of its size; on spheres and tori still one in ten thousand.
 // The postponed leaf's remaining primitives are [cur, end).
 constexpr int kPatchWait = 12;
 
@@ -325,11 +326,8 @@ __device__ __forceinline__ bool traverse_patches(const float4 *__restrict__ node
             if (COUNT) ++nt;
             if (__float_as_uint(a.w) & wrp::kPatchFlag) {
                 float lo[3], hi[3];
-                const uint32_t rec = patch_record(a);
-                wrp::load_patch_box(patches, rec, lo, hi);
-                if (box_entry(r, lo[0], hi[0], lo[1], hi[1], lo[2], hi[2], tmin, t) != __int_as_float(0x7f800000) &&
-                    wrp::meets_hull(patches, rec, make_float3(a.x, a.y, a.z), pr.ox, pr.oy, pr.oz, pr.dx, pr.dy, pr.dz, tmin, t))
-                    ps.pend = i;
+                wrp::load_patch_box(patches, patch_record(a), lo, hi);
+                if (box_entry(r, lo[0], hi[0], lo[1], hi[1], lo[2], hi[2], tmin, t) != __int_as_float(0x7f800000)) ps.pend = i;
                 continue;
             }
             const float4 b = __ldg(tris + 3 * i + 1);
