@@ -372,3 +372,21 @@ def test_guide_learning_rate_is_validated_and_used(wr_lib, cornell):
         nets.append(cornell.guide_params().copy())
     assert all(np.isfinite(i).all() for i in imgs)
     assert not np.array_equal(nets[0], nets[1])
+
+
+def test_training_passes_keep_their_wavefront(wr_lib):
+    """Records are taken in the order of the bounce iterations up to a fixed number, so a training
+    pass's wavefront decides which vertices the network is trained on: 2^21 paths unless the caller
+    chooses, whatever the other passes take."""
+    import json
+    path, _ = golden_scene("cornell")
+    cam = dict(json.load(open(path))["camera"], resolution=[1024, 1024])
+    train = dict(spp=4, num_path_vertices=4, guiding=1, guide_train_spp=4, guide_pass_spp=4, guide_steps=4)
+    with wr_lib.Scene.from_file(path) as sc:
+        sc.set_camera(json.dumps(cam))
+        sc.render(seed=1, **train)
+        assert sc.stats["guide_passes"] == 1 and sc.stats["queue_capacity"] == 1 << 21
+        sc.render(seed=1, queue_capacity=1 << 20, **train)
+        assert sc.stats["queue_capacity"] == 1 << 20
+        sc.render(seed=1, spp=4, num_path_vertices=4, guiding="frozen")
+        assert sc.stats["queue_capacity"] == 1 << 22

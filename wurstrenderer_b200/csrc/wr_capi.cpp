@@ -583,7 +583,9 @@ void render_jobs(wr_scene &s, const std::vector<HostJob> &jobs, const wr_render_
     // Each iteration of the bounce loop ends with a launch tail in which few rays keep the GPU busy;
     // a larger wavefront has fewer of them: 2^20 / 2^21 / 2^22 / 2^23 paths took 47.4 / 44.0 / 42.4 /
     // 41.6 ms for the 1.16M-triangle frame, 95.5 / 93.3 / 90.6 / 98.8 for 24 Cornell jobs.
-    uint32_t capacity = desc.queue_capacity > 0 ? uint32_t(desc.queue_capacity) : (1u << 22);
+    // A pass that collects training records keeps 2^21: records are taken in the order of the bounce
+    // iterations up to a fixed number, so the wavefront decides which vertices a network is trained on.
+    uint32_t capacity = desc.queue_capacity > 0 ? uint32_t(desc.queue_capacity) : po.record ? 1u << 21 : 1u << 22;
     capacity = uint32_t(std::min<unsigned long long>(capacity, std::max<unsigned long long>(total, 1024ull)));
     // A render whose samples all fit the wavefront takes max_nverts - 1 bounce iterations and no
     // more: they are launched one after another with nothing to decide in between, each kernel's
