@@ -421,3 +421,38 @@ def test_patches_with_shared_normals(wr_lib, oracle_lib, tmp_path, family, scale
     assert hits_o > 1000 and 0.85 * hits_o <= hits <= 1.15 * hits_o, (hits, hits_o)
     assert (g != g_o).mean() < 0.05
     assert np.array_equal(occ != 0, g >= 0)
+
+
+def test_deep_trees_in_two_threads(wr_lib, tmp_path):
+    """Two threads, each with a scene whose stacks need more than 48 KB per 256-thread block, one tree
+    deeper than the other: neither takes the other's shared memory away."""
+    import threading
+    from wurstrenderer_b200 import scenes
+    cam = {"pos": [2.5, 0.6, 0.7], "lookat": [0.0, 0.0, 0.0], "up": [0.0, 1.0, 0.0], "fovy": 50.0}
+    paths = []
+    for copies in (1, 8):
+        spec = _nested_quads(47, 0.15)
+        for q in spec.meshes[:47]:
+            for c in range(1, copies):
+                spec.add("%s_%d" % (q.name, c), spec.materials[q.material], q.positions * (1.0 + 0.01 * c), q.triangles)
+        paths.append(scenes.write_spec(str(tmp_path / str(copies)), "nested", spec, cam, [20, 16], 1, 6))
+    scenes_ = [wr_lib.Scene.from_file(p, max_leaf=1) for p in paths]
+    depths = [sc.info["bvh_depth"] for sc in scenes_]
+    assert 46 < depths[0] < depths[1]
+    errors = []
+
+    def job(sc):
+        try:
+            for k in range(300):
+                sc.render(spp=1, seed=k, trace_block=256)
+        except wr_lib.WurstError as e:
+            errors.append(str(e))
+
+    threads = [threading.Thread(target=job, args=(sc,)) for sc in scenes_]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for sc in scenes_:
+        sc.close()
+    assert not errors, errors

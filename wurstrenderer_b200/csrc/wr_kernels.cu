@@ -1219,11 +1219,13 @@ void launch_chained(void (*kernel)(Params...), int grid, int block, size_t smem,
 // (visit counters, for profiled renders)
 enum TraceLaunch { TRACE_EXTEND, TRACE_SHADOW, TRACE_SHADOW_PENDING, TRACE_PAIR };
 
-// bytes of the traversal stacks of a block; more than 48 KB (a 256-thread block on a tree deeper
-// than 46 levels) needs the kernel's consent
+// bytes of the traversal stacks of a block. More than 48 KB (a 256-thread block on a tree deeper than 46
+// levels) needs the kernel's consent, which is the process's and not the scene's: it is given for the
+// deepest tree that any scene may have, so that scenes rendered by other threads never lower it.
 template <class Kernel> size_t stack_bytes(Kernel *kernel, const DevScene &s, int block) {
     const size_t bytes = size_t(s.stack_words) * size_t(block) * 4;
-    if (bytes > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(bytes));
+    if (bytes > 48 * 1024)
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (kMaxStack + 2) * block * 4);
     return bytes;
 }
 
