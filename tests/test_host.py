@@ -212,3 +212,26 @@ def test_obj_number_formats_parse_alike(wr_lib, tmp_path):
     a, b = infos
     assert a["num_triangles"] == b["num_triangles"] == len(tris)
     assert (a["bvh_sah_cost"], a["bvh_nodes"], a["bvh_depth"]) == (b["bvh_sah_cost"], b["bvh_nodes"], b["bvh_depth"])
+
+
+@pytest.mark.parametrize("n", [0, 1, (1 << 20) - 1, (1 << 20) + 1, (1 << 31) - (1 << 20), (1 << 31) - 1])
+def test_long_batches_are_split_whole(tmp_path, n):
+    """The pieces in which a ray batch goes to the device cover it once and in order, up to the largest
+    batch that the interface takes (68 GB of rays, so only the split itself is run here)."""
+    src, exe = tmp_path / "chunks.cpp", tmp_path / "chunks"
+    src.write_text("""
+#include "wr_host.h"
+#include <cstdlib>
+int main() {
+    const size_t n = %dull, chunk = size_t(1) << 20;
+    size_t next = 0, calls = 0;
+    wr::for_chunks(n, chunk, [&](size_t first, size_t count) {
+        if (first != next || count == 0 || count > chunk || ++calls > n / chunk + 1) std::exit(1);
+        next = first + count;
+    });
+    return next == n ? 0 : 1;
+}
+""" % n)
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", os.path.join(ROOT, "wurstrenderer_b200", "csrc"), str(src), "-o",
+                    str(exe)], check=True)
+    assert subprocess.run([str(exe)], timeout=60).returncode == 0

@@ -1142,7 +1142,7 @@ void render_batch(wr_scene &s, const wr_job *jobs, int n, const wr_render_desc *
 
 // One ray batch: the rays go to the device and the wanted answers come back into the caller's arrays,
 // at most kRayChunk rays at a time through buffers that the scene keeps (at most 62 MB).
-constexpr int kRayChunk = 1 << 20;
+constexpr size_t kRayChunk = size_t(1) << 20;
 
 struct RayOutputs {   // host arrays, as RayAnswers
     int *geom = nullptr, *prim = nullptr;
@@ -1156,20 +1156,19 @@ void trace_batch(wr_scene &s, const float *rays, int n, bool any_hit, const RayO
     if (n == 0) return;
     std::lock_guard<std::mutex> lock(s.ray_mutex);
     cudaStream_t st = s.stream;
-    const int chunk = std::min(n, kRayChunk);
-    s.q_rays.alloc(size_t(chunk) * 32);
+    const size_t chunk = std::min(size_t(n), kRayChunk);
+    s.q_rays.alloc(chunk * 32);
     // the answers lie one array after another
     const size_t words = (out.geom ? 1 : 0) + (out.prim ? 1 : 0) + (out.t ? 1 : 0) + (out.uv ? 2 : 0) + (out.normal ? 3 : 0);
-    s.q_answers.alloc(std::max<size_t>(size_t(chunk) * words * 4, 16));
+    s.q_answers.alloc(std::max<size_t>(chunk * words * 4, 16));
     unsigned long long *visits = nullptr;
     if (out.visits) {
         visits = s.q_answers.as<unsigned long long>();
         WR_CUDA(cudaMemsetAsync(visits, 0, 16, st));
     }
     const int sms = sm_count(s);
-    for (int first = 0; first < n; first += chunk) {
-        const int m = std::min(chunk, n - first);
-        WR_CUDA(s.staging->to_device(s.q_rays.p, rays + 8 * size_t(first), size_t(m) * 32, st));
+    wr::for_chunks(size_t(n), chunk, [&](size_t first, size_t m) {
+        WR_CUDA(s.staging->to_device(s.q_rays.p, rays + 8 * first, m * 32, st));
         wrd::RayAnswers a{};
         a.visits = visits;
         struct Back { void *to; const void *from; size_t bytes; };
@@ -1178,8 +1177,8 @@ void trace_batch(wr_scene &s, const float *rays, int n, bool any_hit, const RayO
         auto take = [&](void *host, int per_ray) -> float * {
             if (!host) return nullptr;
             float *dev = next;
-            next += size_t(chunk) * per_ray;
-            back.push_back({static_cast<float *>(host) + size_t(first) * per_ray, dev, size_t(m) * per_ray * 4});
+            next += chunk * per_ray;
+            back.push_back({static_cast<float *>(host) + first * per_ray, dev, m * per_ray * 4});
             return dev;
         };
         a.uv = reinterpret_cast<float2 *>(take(out.uv, 2));   // first: 8-byte aligned
@@ -1191,7 +1190,7 @@ void trace_batch(wr_scene &s, const float *rays, int n, bool any_hit, const RayO
         WR_CUDA(cudaGetLastError());
         for (const Back &b : back) WR_CUDA(s.staging->to_host(b.to, b.from, b.bytes, st));
         // the buffers are free for the next chunk once the copies, which follow the kernel, are done
-    }
+    });
     if (visits) WR_CUDA(cudaMemcpyAsync(out.visits, visits, 16, cudaMemcpyDeviceToHost, st));
     WR_CUDA(cudaStreamSynchronize(st));
 }

@@ -13,6 +13,8 @@
 //   * the thin-lens camera of src/camera/thinlens.h:13-26 and the render list.
 #pragma once
 
+#include <algorithm>
+#include <cstddef>
 #include <cstdint>
 #include <stdexcept>
 #include <string>
@@ -26,6 +28,11 @@ struct Error : std::runtime_error {
     int code;
     Error(int c, const std::string &m) : std::runtime_error(m), code(c) {}
 };
+
+// f(first, count) for [0, n) in pieces of at most `chunk`; in size_t, since a caller's n may be any int
+template <class F> void for_chunks(size_t n, size_t chunk, F f) {
+    for (size_t first = 0; first < n; first += chunk) f(first, std::min(chunk, n - first));
+}
 
 // status codes are the WR_* values of include/wurst_b200.h
 struct Material {          // TwoSided(inner) material of one surface mesh
