@@ -46,7 +46,7 @@ typedef struct wr_render_desc {
     int grid_shade;          /* persistent blocks of shade / raygen; 0 = occupancy-derived */
     int use_graph;           /* 1: the whole render is one CUDA-graph launch (while-loop node over the
                                 bounce iterations), or, when all its samples fit the wavefront, a
-                                fixed chain of overlapping launches; 0: host-driven launches */
+                                chain of overlapping launches; 0: host-driven launches */
     int profile;             /* 0: off; 1: per-kernel CUDA-event timing (plain launches, extend and
                                 shadow rays in separate kernels); 2: timing + traversal counters
                                 (node visits, triangle tests); 3: as 2 with the fused schedule of

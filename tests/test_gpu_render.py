@@ -354,3 +354,24 @@ def test_images_reach_the_host_whole(wr_lib, res):
             assert np.allclose(im, want[k], rtol=1e-9, atol=1e-12)
     for sc in scenes_:
         sc.close()
+
+
+@pytest.mark.parametrize("integrator", ["nextevent_path_tracer", "primitive_path_tracer", "light_splatting"])
+@pytest.mark.parametrize("nverts", [21, 22, 41, 64, 65])
+def test_renders_end_with_their_paths(wr_lib, tmp_path, nverts, integrator):
+    """A floor under the open sky: paths end after a few vertices, however many were asked for, and the
+    render does not go on with an empty wavefront; a smaller wavefront makes it one graph."""
+    from wurstrenderer_b200 import scenes
+    spec = scenes.SceneSpec()
+    p, t = scenes.quad((-3.0, 0.0, -3.0), (-3.0, 0.0, 3.0), (3.0, 0.0, 3.0), (3.0, 0.0, -3.0))
+    spec.add("floor", scenes.Material("m_floor", kd=(0.5, 0.5, 0.5)), p, t)
+    p, t = scenes.quad((-0.5, 4.0, -0.5), (0.5, 4.0, -0.5), (0.5, 4.0, 0.5), (-0.5, 4.0, 0.5))
+    spec.add("light", scenes.Material("m_light", ke=(9.0, 9.0, 9.0)), p, t)
+    cam = {"pos": [0.0, 3.0, 6.0], "lookat": [0.0, 0.0, 0.0], "up": [0.0, 1.0, 0.0], "fovy": 50.0}
+    path = scenes.write_spec(str(tmp_path), "open", spec, cam, [64, 48], 1, 10)
+    kw = dict(spp=2, num_path_vertices=nverts, seed=5, integrator=integrator)
+    with wr_lib.Scene.from_file(path) as sc:
+        image = sc.render(**kw)
+        assert sc.stats["iterations"] <= 21
+        graph = sc.render(queue_capacity=1024, **kw)
+    assert image.any() and np.allclose(image, graph, rtol=1e-9, atol=1e-12)
