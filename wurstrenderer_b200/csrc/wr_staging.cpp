@@ -90,12 +90,13 @@ cudaError_t Staging::share(int k, int parts, bool up, char *host, char *dev, siz
         } else {
             e = cudaMemcpyAsync(buf[b], dev + i * kPiece, size_of(i), cudaMemcpyDeviceToHost, st);
         }
-        if (e != cudaSuccess) break;
-        flight[b] = {i, true};
-        e = cudaEventRecord(ev[b], st);
+        if (e == cudaSuccess) e = cudaEventRecord(ev[b], st);
+        if (e == cudaSuccess) flight[b] = {i, true};
     }
     finish(b);       // the older piece first
     finish(b ^ 1);
+    // after an error a piece without an event may still be on the bus: its buffer is free with the stream
+    if (e != cudaSuccess) cudaStreamSynchronize(st);
     for (cudaEvent_t v : ev)
         if (v) cudaEventDestroy(v);
     return e;
