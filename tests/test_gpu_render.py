@@ -375,3 +375,16 @@ def test_renders_end_with_their_paths(wr_lib, tmp_path, nverts, integrator):
         assert sc.stats["iterations"] <= 21
         graph = sc.render(queue_capacity=1024, **kw)
     assert image.any() and np.allclose(image, graph, rtol=1e-9, atol=1e-12)
+
+
+def test_images_of_a_long_session_reach_the_host_whole(wr_lib):
+    """Frame after frame into fresh arrays, through the driver's copies and the staged ones that follow."""
+    import json
+    path, _ = golden_scene("cornell")
+    cam = dict(json.load(open(path))["camera"], resolution=[1023, 511])
+    with wr_lib.Scene.from_file(path) as sc:
+        sc.set_camera(json.dumps(cam))
+        images = [sc.render(spp=1, seed=6) for _ in range(9)]
+    assert images[0].any()
+    for im in images[1:]:
+        assert np.allclose(im, images[0], rtol=1e-9, atol=1e-12)

@@ -141,3 +141,29 @@ int main() {
     CHECK(pinned.empty() && early_frees == 0);
 }
 """ % (fail, way, "host.data(), dev.data(), n, nullptr" if way == "to_host" else "dev.data(), a.data(), n, nullptr"))
+
+
+def test_few_large_copies_need_no_buffers(tmp_path):
+    """A program that copies little never pays for the staging buffers; one that goes on, or copies much
+    at once, gets them, and they are given back with the last holder."""
+    run_program(tmp_path, r"""
+int main() {
+    for (size_t mb : {3, 20, 64, 65}) {
+        host_allocs = 0;
+        auto s = wr::Staging::shared();
+        const size_t n = mb << 20;
+        auto a = bytes_of(n, unsigned(mb));
+        std::vector<unsigned char> dev(n), host(n);
+        size_t copied = 0;
+        for (int k = 0; k < 30 && copied < (size_t(200) << 20); ++k) {
+            const bool up = k % 2 == 0;
+            CHECK((up ? s->to_device(dev.data(), a.data(), n, nullptr) : s->to_host(host.data(), dev.data(), n, nullptr)) == cudaSuccess);
+            CHECK(up ? dev == a : host == a);
+            copied += n;
+            CHECK(host_allocs == (copied > (size_t(64) << 20) ? 1 : 0));
+        }
+        s.reset();
+        CHECK(pinned.empty() && early_frees == 0);
+    }
+}
+""")

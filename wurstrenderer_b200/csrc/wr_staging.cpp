@@ -27,9 +27,12 @@ Staging::~Staging() {
     if (pinned_) cudaFreeHost(pinned_);
 }
 
-// makes the buffers and threads once; false when either cannot be had
-bool Staging::prepare() {
+// makes the buffers and threads once; false while the large copies so far, `bytes` more with this one, are
+// not worth them, and when they cannot be had
+bool Staging::prepare(size_t bytes) {
     if (pinned_) return true;
+    copied_ += bytes;
+    if (copied_ <= kPrepareAfter) return false;
     void *p = nullptr;
     if (cudaHostAlloc(&p, 2 * kThreads * kPiece, cudaHostAllocPortable) != cudaSuccess) {
         cudaGetLastError();   // out of pinned memory: the driver copies
@@ -117,7 +120,7 @@ cudaError_t Staging::copy(bool up, char *host, char *dev, size_t bytes, cudaStre
         }
     }
     std::unique_lock<std::mutex> lock(use_, std::defer_lock);
-    if (direct || !lock.try_lock() || !prepare()) return cudaMemcpyAsync(to, from, bytes, kind, st);
+    if (direct || !lock.try_lock() || !prepare(bytes)) return cudaMemcpyAsync(to, from, bytes, kind, st);
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return e;

@@ -5,7 +5,10 @@
 // most of it first touches of a fresh array's pages. Here a few threads share a copy: each stages
 // its pieces through pinned memory, one piece on the bus while another is copied in host memory
 // (0.5 and 4 ms; a million rays' queries 13.3 -> 6.4 ms, 200,003 guide points 2.3 -> 1.2).
-// Pinned memory and copies below kDirectBytes go straight to the driver.
+// Pinned memory and copies below kDirectBytes go straight to the driver, and so do the first
+// kPrepareAfter bytes of large copies: the buffers and threads take 15 ms to make, which a program that
+// loads a scene, renders a frame and ends would pay for nothing (400x300 from a fresh scene: 4.6 ms by
+// the driver, 18 with them), and staging saves 0.05 to 0.4 ms a MB.
 #pragma once
 
 #include <condition_variable>
@@ -22,8 +25,8 @@ namespace wr {
 
 class Staging {
 public:
-    // the process's staging buffers and threads (16 MB and up to 7 threads, made by the first large
-    // copy), shared by the scenes that hold the pointer and given back with the last of them
+    // the process's staging buffers and threads (16 MB and up to 7 threads, made when enough has been
+    // copied), shared by the scenes that hold the pointer and given back with the last of them
     static std::shared_ptr<Staging> shared();
     ~Staging();
 
@@ -36,13 +39,15 @@ private:
     static constexpr int kThreads = 8;                   // the calling thread and up to seven others
     static constexpr size_t kPiece = size_t(1) << 20;    // staged at a time; two per thread
     static constexpr size_t kDirectBytes = size_t(2) << 20;
+    static constexpr size_t kPrepareAfter = size_t(64) << 20;
 
     cudaError_t copy(bool up, char *host, char *dev, size_t bytes, cudaStream_t st);
     cudaError_t share(int k, int parts, bool up, char *host, char *dev, size_t bytes, cudaStream_t st, int device);
-    bool prepare();
+    bool prepare(size_t bytes);
     void work(int k);
 
     std::mutex use_;                     // one copy at a time; another thread's goes to the driver
+    size_t copied_ = 0;                  // bytes of large copies before the buffers were made
     char *pinned_ = nullptr;
     std::vector<std::thread> threads_;
     std::mutex m_;
