@@ -456,3 +456,34 @@ def test_deep_trees_in_two_threads(wr_lib, tmp_path):
     for sc in scenes_:
         sc.close()
     assert not errors, errors
+
+
+@pytest.mark.parametrize("n", [1, 2, 2730, 2731, 3276, 3277, 3278])
+def test_short_batches_answer_like_long_ones(wr_lib, n):
+    """Batches around the size up to which all answers come back in one copy."""
+    path, _ = golden_scene("cornell")
+    rays = np.load("%s/%s_rays.npy" % (GOLDEN, "cornell"))
+    rays = rays[np.arange(40000) % len(rays)]
+    with wr_lib.Scene.from_file(path) as sc:
+        whole = sc.trace_closest(rays) + sc.trace_hits(rays)
+        part = sc.trace_closest(rays[5:5 + n]) + sc.trace_hits(rays[5:5 + n])
+    for a, b in zip(whole, part):
+        assert np.array_equal(a[5:5 + n], b)
+
+
+def test_one_ray_is_one_round_trip(wr_lib):
+    """A closest-hit query of one ray returns four arrays and an occlusion query one, but both copy to the
+    host once: a copy per array takes twice as long as the occlusion query."""
+    import time
+    path, _ = golden_scene("cornell")
+    ray = np.load("%s/%s_rays.npy" % (GOLDEN, "cornell"))[:1]
+    times = {"closest": [], "occluded": []}
+    with wr_lib.Scene.from_file(path) as sc:
+        for k in range(400):
+            for name, query in (("closest", sc.trace_closest), ("occluded", sc.trace_occluded)):
+                t = time.perf_counter()
+                query(ray)
+                if k >= 50:
+                    times[name].append(time.perf_counter() - t)
+    closest, occluded = np.median(times["closest"]), np.median(times["occluded"])
+    assert closest < 1.6 * occluded, (closest, occluded)
