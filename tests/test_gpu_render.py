@@ -388,3 +388,23 @@ def test_images_of_a_long_session_reach_the_host_whole(wr_lib):
     assert images[0].any()
     for im in images[1:]:
         assert np.allclose(im, images[0], rtol=1e-9, atol=1e-12)
+
+
+@pytest.mark.parametrize("guiding", [0, "frozen"])
+def test_a_render_that_does_not_fit_leaves_the_scene_usable(wr_lib, guiding):
+    """A wavefront of 2^30 paths (232 GB) fails with an out-of-memory error; the renders after it, of the
+    size before it and of others, are what they were."""
+    import json
+    path, _ = golden_scene("cornell")
+    camera = json.load(open(path))["camera"]
+    with wr_lib.Scene.from_file(path) as sc:
+        before = sc.render(spp=4, seed=2, guiding=guiding)
+        sc.set_camera(json.dumps(dict(camera, resolution=[1024, 1024])))
+        with pytest.raises(wr_lib.WurstError) as e:
+            sc.render(spp=1024, seed=2, queue_capacity=1 << 30, guiding=guiding)
+        assert e.value.status == 6     # WR_ERR_OUT_OF_MEMORY
+        sc.set_camera(json.dumps(camera))
+        after = sc.render(spp=4, seed=2, guiding=guiding)
+        small = sc.render(spp=4, seed=2, queue_capacity=1024, guiding=guiding)
+    assert before.any() and np.allclose(after, before, rtol=1e-9, atol=1e-12)
+    assert np.allclose(small, before, rtol=1e-9, atol=1e-12)

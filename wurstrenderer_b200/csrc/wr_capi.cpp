@@ -62,7 +62,12 @@ struct DevBuf {
     void alloc(size_t n) {
         if (n <= bytes && p) return;
         release();
-        WR_CUDA(cudaMalloc(&p, std::max<size_t>(n, 16)));
+        const cudaError_t e = cudaMalloc(&p, std::max<size_t>(n, 16));
+        if (e != cudaSuccess) {
+            p = nullptr;
+            cudaGetLastError();   // reported here, not by the next launch's check
+        }
+        WR_CUDA(e);
         bytes = n;
     }
     template <typename T> T *as() const { return static_cast<T *>(p); }
@@ -100,9 +105,7 @@ struct wr_scene {
     DevBuf q_rays, q_answers;   // ray batches: one chunk of rays and its answers
     std::vector<float> q_host;  // a short batch's answers on their way to the caller's arrays
     std::mutex ray_mutex;       // one batch at a time uses them
-    uint32_t w_guide_capacity = 0, w_record_capacity = 0;
-    uint32_t w_capacity = 0;
-    size_t w_npix = 0;
+    uint32_t w_record_capacity = 0;
     std::shared_ptr<wr::Staging> staging = wr::Staging::shared();
     uint32_t *pinned = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -486,27 +489,23 @@ wrd::DevCamera make_camera(const wr::Camera &c) {
     return d;
 }
 
+// The wavefront's buffers, grown where they are too small. What is there is asked of each buffer, so a
+// call after one that ran out of memory finds what that one left.
 void ensure_wave(wr_scene &s, uint32_t capacity, size_t npix) {
-    if (s.w_capacity != capacity) {
-        for (int p = 0; p < 2; ++p) {
-            s.w_o[p].alloc(size_t(capacity) * 16);
-            s.w_d[p].alloc(size_t(capacity) * 16);
-            s.w_thr[p].alloc(size_t(capacity) * 16);
-            s.w_meta[p].alloc(size_t(capacity) * 4);
-        }
-        s.w_hit.alloc(size_t(capacity) * 16);
-        s.w_sho.alloc(size_t(capacity) * 2 * 16);
-        s.w_shd.alloc(size_t(capacity) * 2 * 16);
-        s.w_shc.alloc(size_t(capacity) * 2 * 16);
-        s.w_ctr.alloc(wrd::CTR_COUNT * 4);
-        s.w_sample.alloc(8);
-        s.w_capacity = capacity;
+    for (int p = 0; p < 2; ++p) {
+        s.w_o[p].alloc(size_t(capacity) * 16);
+        s.w_d[p].alloc(size_t(capacity) * 16);
+        s.w_thr[p].alloc(size_t(capacity) * 16);
+        s.w_meta[p].alloc(size_t(capacity) * 4);
     }
-    if (s.w_npix != npix) {
-        s.w_film.alloc(npix * 6 * 8);
-        s.w_out.alloc(npix * 3 * 8);
-        s.w_npix = npix;
-    }
+    s.w_hit.alloc(size_t(capacity) * 16);
+    s.w_sho.alloc(size_t(capacity) * 2 * 16);
+    s.w_shd.alloc(size_t(capacity) * 2 * 16);
+    s.w_shc.alloc(size_t(capacity) * 2 * 16);
+    s.w_ctr.alloc(wrd::CTR_COUNT * 4);
+    s.w_sample.alloc(8);
+    s.w_film.alloc(npix * 6 * 8);
+    s.w_out.alloc(npix * 3 * 8);
 }
 
 struct HostJob {
@@ -527,13 +526,11 @@ struct PassOpts {
 };
 
 void ensure_guide_wave(wr_scene &s, uint32_t capacity, uint32_t record_capacity) {
-    if (s.w_guide_capacity != capacity) {
-        s.w_rec[0].alloc(size_t(capacity) * 4);
-        s.w_rec[1].alloc(size_t(capacity) * 4);
-        s.w_lobes.alloc(size_t(capacity) * wrg::kPackedChunks * 16);
-        s.w_guide_capacity = capacity;
-    }
+    s.w_rec[0].alloc(size_t(capacity) * 4);
+    s.w_rec[1].alloc(size_t(capacity) * 4);
+    s.w_lobes.alloc(size_t(capacity) * wrg::kPackedChunks * 16);
     if (record_capacity > s.w_record_capacity) {
+        s.w_record_capacity = 0;
         s.w_records.alloc(size_t(record_capacity) * wrg::kRecordFloat4 * 16);
         s.w_record_capacity = record_capacity;
     }

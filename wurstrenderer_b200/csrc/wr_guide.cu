@@ -689,9 +689,10 @@ __global__ void k_guide_init(GuideNet g, uint32_t seed) {
 namespace wrg {
 
 static void check(cudaError_t e, const char *what) {
-    if (e != cudaSuccess)
-        throw wr::Error(e == cudaErrorMemoryAllocation ? WR_ERR_OUT_OF_MEMORY : WR_ERR_CUDA,
-                        std::string(what) + ": " + cudaGetErrorString(e));
+    if (e == cudaSuccess) return;
+    cudaGetLastError();   // reported here, not by the next launch's check
+    throw wr::Error(e == cudaErrorMemoryAllocation ? WR_ERR_OUT_OF_MEMORY : WR_ERR_CUDA,
+                    std::string(what) + ": " + cudaGetErrorString(e));
 }
 
 void guide_alloc(GuideNet &g) {
