@@ -41,7 +41,9 @@ typedef struct wr_render_desc {
     int num_path_vertices;   /* <= 0 takes "num_path_vertices" of the render entry (default 10) */
     unsigned int seed;       /* selects the random streams; 0 is a valid seed */
     int render_index;        /* which "render" entry supplies the defaults */
-    int queue_capacity;      /* wavefront slots; 0 = default (tuned) */
+    int queue_capacity;      /* wavefront slots (paths in flight), 216 bytes each and 88 more in guided passes;
+                                0 = 2^22, or 2^21 where those do not fit the device's free memory and in
+                                passes that collect training records; never more than the render's samples */
     int grid_trace;          /* persistent blocks of the traversal kernels; 0 = occupancy-derived */
     int grid_shade;          /* persistent blocks of shade / raygen; 0 = occupancy-derived */
     int use_graph;           /* 1: the whole render is one CUDA-graph launch (while-loop node over the

@@ -408,3 +408,32 @@ def test_a_render_that_does_not_fit_leaves_the_scene_usable(wr_lib, guiding):
         small = sc.render(spp=4, seed=2, queue_capacity=1024, guiding=guiding)
     assert before.any() and np.allclose(after, before, rtol=1e-9, atol=1e-12)
     assert np.allclose(small, before, rtol=1e-9, atol=1e-12)
+
+
+@pytest.mark.parametrize("guiding,left_mb", [(0, 750), ("frozen", 1000)])
+def test_the_default_wavefront_gives_way(wr_lib, guiding, left_mb):
+    """Beside another user of the device's memory, a render whose default wavefront does not fit takes
+    half of it, which did fit before the default was doubled; a wavefront that the caller names does not."""
+    import json
+    import torch
+    path, _ = golden_scene("cornell")
+    camera = json.load(open(path))["camera"]
+    kw = dict(spp=4, num_path_vertices=4, seed=2, guiding=guiding)
+    with wr_lib.Scene.from_file(path) as sc:
+        sc.render(spp=1, guiding=guiding)
+        sc.set_camera(json.dumps(dict(camera, resolution=[1024, 1024])))
+        other = torch.empty(torch.cuda.mem_get_info()[0] - (left_mb << 20), dtype=torch.uint8, device="cuda")
+        try:
+            tight = sc.render(**kw)
+            assert sc.stats["queue_capacity"] == 1 << 21
+            again = sc.render(**kw)
+            with pytest.raises(wr_lib.WurstError) as e:
+                sc.render(queue_capacity=1 << 22, **kw)
+            assert e.value.status == 6     # WR_ERR_OUT_OF_MEMORY
+        finally:
+            del other
+            torch.cuda.empty_cache()
+        named = sc.render(queue_capacity=1 << 22, **kw)
+        assert sc.stats["queue_capacity"] == 1 << 22
+    assert tight.any() and np.allclose(again, tight, rtol=1e-9, atol=1e-12)
+    assert np.allclose(named, tight, rtol=1e-9, atol=1e-12)

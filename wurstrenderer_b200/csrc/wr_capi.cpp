@@ -106,6 +106,7 @@ struct wr_scene {
     std::vector<float> q_host;  // a short batch's answers on their way to the caller's arrays
     std::mutex ray_mutex;       // one batch at a time uses them
     uint32_t w_record_capacity = 0;
+    uint32_t w_default = 1u << 22;   // wavefront where the caller names none; halved once when it does not fit
     std::shared_ptr<wr::Staging> staging = wr::Staging::shared();
     uint32_t *pinned = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -537,6 +538,14 @@ void ensure_guide_wave(wr_scene &s, uint32_t capacity, uint32_t record_capacity)
     s.w_rec_count.alloc(16);
 }
 
+// Gives the buffers back that a wavefront which did not fit has taken; a film that further passes add to
+// and records stay.
+void release_wave(wr_scene &s) {
+    for (int p = 0; p < 2; ++p)
+        for (DevBuf *b : {&s.w_o[p], &s.w_d[p], &s.w_thr[p], &s.w_meta[p], &s.w_rec[p]}) b->release();
+    for (DevBuf *b : {&s.w_hit, &s.w_sho, &s.w_shd, &s.w_shc, &s.w_lobes}) b->release();
+}
+
 int integrator_of(const std::string &name) {
     if (name.empty() || name == "nextevent_path_tracer") return wrd::INTEGRATOR_NEE;
     if (name == "primitive_path_tracer") return wrd::INTEGRATOR_PRIMITIVE;
@@ -583,8 +592,23 @@ void render_jobs(wr_scene &s, const std::vector<HostJob> &jobs, const wr_render_
     // 41.6 ms for the 1.16M-triangle frame, 95.5 / 93.3 / 90.6 / 98.8 for 24 Cornell jobs.
     // A pass that collects training records keeps 2^21: records are taken in the order of the bounce
     // iterations up to a fixed number, so the wavefront decides which vertices a network is trained on.
-    uint32_t capacity = desc.queue_capacity > 0 ? uint32_t(desc.queue_capacity) : po.record ? 1u << 21 : 1u << 22;
+    uint32_t capacity = desc.queue_capacity > 0 ? uint32_t(desc.queue_capacity) : po.record ? 1u << 21 : s.w_default;
     capacity = uint32_t(std::min<unsigned long long>(capacity, std::max<unsigned long long>(total, 1024ull)));
+    const bool guided = po.guide || po.record;
+    auto ensure = [&]() {
+        ensure_wave(s, capacity, total_pix);
+        if (guided) ensure_guide_wave(s, capacity, po.record_capacity);
+    };
+    // 2^22 paths take 906 MB, 1275 with a network's lobes: where the default does not fit beside the
+    // device's other users it gives way to 2^21, half of that.
+    try {
+        ensure();
+    } catch (const Error &e) {
+        release_wave(s);
+        if (e.code != WR_ERR_OUT_OF_MEMORY || desc.queue_capacity > 0 || capacity <= (1u << 21)) throw;
+        s.w_default = capacity = 1u << 21;
+        ensure();
+    }
     // A render whose samples all fit the wavefront takes max_nverts - 1 bounce iterations and no
     // more: they are launched one after another with little to decide in between (`look` below),
     // each kernel's set-up overlapping the one before it. Building and instantiating a graph costs the host more
@@ -593,7 +617,6 @@ void render_jobs(wr_scene &s, const std::vector<HostJob> &jobs, const wr_render_
     // 1.31, 1.24). Longer renders, whose number of iterations only the device knows, are one graph;
     // overlapping the launches inside it changes nothing (44.0 against 43.9 ms for the 1M frame).
     const bool one_wave = total <= capacity && max_nverts <= 64;
-    ensure_wave(s, capacity, total_pix);
     cudaStream_t st = s.stream;
 
     wrk::WaveBuffers b{};
@@ -612,9 +635,7 @@ void render_jobs(wr_scene &s, const std::vector<HostJob> &jobs, const wr_render_
     b.sample_next = s.w_sample.as<unsigned long long>();
     b.capacity = capacity;
     b.shadow_capacity = 2 * capacity;
-    const bool guided = po.guide || po.record;
     if (guided) {
-        ensure_guide_wave(s, capacity, po.record_capacity);
         b.rec[0] = s.w_rec[0].as<uint32_t>();
         b.rec[1] = s.w_rec[1].as<uint32_t>();
         b.lobes = s.w_lobes.as<uint4>();
