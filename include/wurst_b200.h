@@ -73,7 +73,8 @@ typedef struct wr_render_desc {
     float guide_clamp;       /* loss weights are clamped at guide_clamp x their mean over the pass;
                                 0 = 1000, < 0 = no clamp */
     int fetch_threshold;     /* traversal: a warp hands new rays to its idle lanes when fewer than this
-                                many of its 32 lanes are still traversing; 1..32, 0 = 20 */
+                                many of its 32 lanes are still traversing; 1..32, 0 = 12, or 20 in
+                                scenes with Phong patches */
     int max_iterations;      /* debugging: lowers the wavefront's iteration bound (0 = the bound derived
                                 from the work, (waves + 2) * (num_path_vertices + 2) + 64). A render
                                 that has not drained when its bound is reached stops and returns

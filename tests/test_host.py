@@ -235,3 +235,23 @@ int main() {
     subprocess.run(["g++", "-std=c++17", "-O1", "-I", os.path.join(ROOT, "wurstrenderer_b200", "csrc"), str(src), "-o",
                     str(exe)], check=True)
     assert subprocess.run([str(exe)], timeout=60).returncode == 0
+
+
+def test_autotuner_tries_every_other_fetch_threshold(tmp_path):
+    """The autotuner's thresholds do not repeat the scene's default and do not miss the other kind's."""
+    src, exe = tmp_path / "fetch.cpp", tmp_path / "fetch"
+    src.write_text("""
+#include "wr_host.h"
+#include <cstdio>
+int main() {
+    for (bool patches : {false, true}) {
+        std::printf("%d:", wr::default_fetch(patches));
+        for (int th : wr::fetch_candidates(patches)) std::printf(" %d", th);
+        std::printf("\\n");
+    }
+}
+""")
+    subprocess.run(["g++", "-std=c++17", "-O1", "-I", os.path.join(ROOT, "wurstrenderer_b200", "csrc"), str(src), "-o",
+                    str(exe)], check=True)
+    out = subprocess.run([str(exe)], capture_output=True, text=True, check=True).stdout.split("\n")
+    assert out[:2] == ["12: 16 20 24 28", "20: 12 16 24 28"]

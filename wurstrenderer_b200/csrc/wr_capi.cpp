@@ -650,10 +650,7 @@ void render_jobs(wr_scene &s, const std::vector<HostJob> &jobs, const wr_render_
     r.guide_sms = sms;
     if (desc.fetch_threshold < 0 || desc.fetch_threshold > 32)
         throw Error(WR_ERR_INVALID_ARGUMENT, "fetch_threshold must be 0..32");
-    // lanes still traversing below which a warp takes new rays: 8 / 12 / 16 / 20 / 24 measured 41.9 / 41.8 /
-    // 41.9 / 42.3 / 43.1 ms for the 1.16M-triangle frame, but 12 / 20 / 24 14.1 / 13.9 / 14.0 for 56,000
-    // patches, where the refill interrupts gathered patch tests
-    r.fetch_min = desc.fetch_threshold > 0 ? desc.fetch_threshold : s.dev.patches ? 20 : 12;
+    r.fetch_min = desc.fetch_threshold > 0 ? desc.fetch_threshold : wr::default_fetch(s.dev.patches != nullptr);
     r.num_jobs = int(table.size());
     r.job0 = table[0];
     r.nee_only = 1;
@@ -1514,7 +1511,7 @@ wr_render_desc tune_knobs(wr_scene &s, wr_render_desc cur, Probe probe, double *
         if (t < bt * kTuneMargin) { bt = t; cur = d; }
     }
     // 4) dynamic ray fetching threshold
-    for (int th : {12, 16, 24, 28}) {
+    for (int th : wr::fetch_candidates(s.dev.patches != nullptr)) {
         wr_render_desc d = cur;
         d.fetch_threshold = th;
         const double t = trial(d);

@@ -34,6 +34,20 @@ template <class F> void for_chunks(size_t n, size_t chunk, F f) {
     for (size_t first = 0; first < n; first += chunk) f(first, std::min(chunk, n - first));
 }
 
+// Dynamic ray fetching: lanes still traversing below which a warp takes new rays. 8 / 12 / 16 / 20 / 24
+// measured 41.9 / 41.8 / 42.0 / 42.3 / 43.1 ms for the 1.16M-triangle frame, 7.82 / 7.80 / 7.82 / 7.84 /
+// 7.93 for a sky scene, 19.6 / 19.6 / 19.7 / 20.0 / 20.1 for the door room, 8.86 / 8.76 / 8.75 / 8.75 / 8.76
+// for a Cornell box; with Phong patches, where the refill interrupts gathered patch tests, 17.9 / 17.4 /
+// 17.3 / 17.1 / 17.0 at 4 spp and 56.8 / 54.5 / 53.6 / 52.5 / 51.9 at 16.
+inline int default_fetch(bool patches) { return patches ? 20 : 12; }
+// what the autotuner tries beside that default
+inline std::vector<int> fetch_candidates(bool patches) {
+    std::vector<int> v;
+    for (int th : {12, 16, 20, 24, 28})
+        if (th != default_fetch(patches)) v.push_back(th);
+    return v;
+}
+
 // status codes are the WR_* values of include/wurst_b200.h
 struct Material {          // TwoSided(inner) material of one surface mesh
     float kd[3] = {0, 0, 0};

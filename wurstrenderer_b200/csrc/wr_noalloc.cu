@@ -200,7 +200,7 @@ extern "C" int wr_render_device_noalloc(wr_scene *scene, const wr_render_desc *d
     r.grid_shade = desc.grid_shade > 0 ? desc.grid_shade : sms * std::max(1, wrk::shade_occupancy());
     if (desc.fetch_threshold < 0 || desc.fetch_threshold > 32)
         return fail(WR_ERR_INVALID_ARGUMENT, "fetch_threshold must be 0..32");
-    r.fetch_min = desc.fetch_threshold > 0 ? desc.fetch_threshold : v.dev.patches ? 20 : 12;   // as wr_render_device
+    r.fetch_min = desc.fetch_threshold > 0 ? desc.fetch_threshold : wr::default_fetch(v.dev.patches != nullptr);
     r.has_cond = 0;
     r.prof = nullptr;
 
