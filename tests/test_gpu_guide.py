@@ -390,3 +390,16 @@ def test_training_passes_keep_their_wavefront(wr_lib):
         assert sc.stats["queue_capacity"] == 1 << 20
         sc.render(seed=1, spp=4, num_path_vertices=4, guiding="frozen")
         assert sc.stats["queue_capacity"] == 1 << 22
+
+
+@pytest.mark.parametrize("nverts", [3, 10, 24])
+def test_frozen_one_wave_renders_match_graphs(cornell, nverts):
+    """A guided render whose samples fit the wavefront is a chain of launches with the inference kernel
+    between them; the same samples through a smaller wavefront are one graph."""
+    cornell.guide_set_params(_net(np.random.default_rng(17)))
+    kw = dict(spp=3, num_path_vertices=nverts, seed=4, guiding="frozen")
+    chained = cornell.render(**kw)
+    graph = cornell.render(queue_capacity=1024, **kw)
+    plain = cornell.render(use_graph=False, queue_capacity=1024, **kw)
+    assert chained.any() and np.allclose(chained, graph, rtol=1e-9, atol=1e-12)
+    assert np.allclose(plain, graph, rtol=1e-9, atol=1e-12)
