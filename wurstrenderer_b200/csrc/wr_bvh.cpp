@@ -56,7 +56,7 @@ struct TmpNode {
 
 constexpr int kBins = 32;
 constexpr uint32_t kMaxLeafHard = 16;   // 4-bit count field
-constexpr int kDepthBudget = 60;         // traversal stack holds 64 entries
+constexpr int kDepthBudget = 60;         // below the deepest tree that a scene may have (wrd::kMaxStack)
 constexpr uint32_t kParallelRange = 1u << 18;   // ranges at least this long are binned by several threads
 constexpr uint32_t kChunk = 1u << 16;           // primitives per thread at least
 constexpr uint32_t kSpawnRange = 1u << 13;      // subtrees at least this large may get a thread

@@ -14,10 +14,10 @@
 //                   1M-triangle workload)
 //
 // Leaves hold one or two triangles. Every inner node splits at the first differing key bit
-// of its range, so the depth is at most 63 (key bits + 1) and the 64-entry
-// traversal stack always suffices. The result replaces Embree's BVH build
-// (src/accel/embreeaccel.h:466-469) when a scene is created with the device builder;
-// the default remains the host binned-SAH build, whose trees traverse faster.
+// of its range, so the depth is at most 63 (key bits + 1), below the deepest tree that
+// a scene may have (wrd::kMaxStack; the traversal stack holds the tree's depth + 2
+// entries). The result replaces Embree's BVH build (src/accel/embreeaccel.h:466-469) when a
+// scene is created with the device builder; the default remains the host binned-SAH build, whose trees traverse faster.
 
 #include <cstdint>
 #include <cstring>

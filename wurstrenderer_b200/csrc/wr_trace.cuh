@@ -207,7 +207,7 @@ struct TraceStack {
 // leaf pass the warp returns when fewer than `min_active` of its lanes are still traversing, so that
 // the caller can hand new rays to the finished ones. The votes only steer the schedule; each lane's
 // result does not depend on other lanes. kLeafWait = 1 / 4 / 8 / 12 measured 45.3 / 43.8 / 44.0 /
-// 44.7 ms for the 1.16M-triangle frame.
+// 44.7 ms for the 1.16M-triangle frame; 1 / 4 1.124 / 1.136 for a small frame of the Cornell box.
 constexpr int kLeafWait = 4;
 
 template <bool ANY_HIT, bool UV, bool COUNT>
@@ -273,7 +273,8 @@ __device__ __forceinline__ bool traverse_steps(const float4 *__restrict__ nodes,
 // different places in it thrashed the instruction cache. Here a lane whose patch passes its own box
 // holds it (`pend`) and waits, descending further where it can, until kPatchWait lanes of the warp hold
 // one or none can do anything else: 27.0 -> 18.9 ms for a frame of 56,000 patches (kPatchWait 1 / 8 / 12 /
-// 16 / 20: 19.6 / 18.7 / 18.9 / 18.8 / 19.0), 16.9 with the registers that the fused kernel then gives it.
+// 16 / 20: 19.6 / 18.7 / 18.9 / 18.8 / 19.0; 12 lies amid the values that differ by no more than runs do),
+// 16.9 with the registers that the fused kernel then gives it.
 // Nothing but its own box may keep a ray from a patch's FP64 test: the test also accepts points off the
 // ray, and they are part of the answer. Where two vertex normals equal the face normal, or on a cylinder,
 // the pencil of conics degenerates and a third of all accepted points lie outside the patch's convex
